@@ -988,41 +988,49 @@ k_sweep_bwd(int32_t l0, int32_t l1, const int32_t *__restrict__ cells,
 }
 
 // ---------------------------------------------------------------------------
-// Persistent chunked sweeps, warp-specialised.
+// Persistent chunked sweeps, one block per SM.
 //
-// The cells are split into chunks, one per block and one block per SM
-// (cooperative launch).  A block walks the levels of its chunk in increasing
-// order; a level with more cells than the block has lane groups takes several
-// passes, and every (level, pass) is one work item.  The block's warps have
-// two roles:
+// The cells are split into chunks, one per block (cooperative launch).  A
+// chunk's positions are level-major; a level's positions are cut into items
+// of 32 / L cells, and the items of the chunk, in level order, go to the
+// block's warps in turn.  A warp sweeps its item alone: lane h of a cell's L
+// lanes owns the records h, h + L, ... of the cell.  Before its turn it reads
+// everything of the item that no sweep writes -- the states of the cells and
+// of their neighbours, the faces, Diag, the right-hand side -- and forms what
+// they give (the neighbour-state half of FluxLUSGS3D, the diagonal term's
+// reciprocal) in registers; the dependent chain then holds only the
+// neighbours' increments, the rest of FluxLUSGS3D, the ordered sums, the
+// quotients and the limiter.  While one warp runs its chain, the others read
+// ahead or store: with kSweepWarps warps and a few items per level, a warp
+// reads several levels ahead of its turn.
 //
-//  * producer warps, in kWsTeams teams taking the items in turn, read what an
-//    item's cells need that no sweep writes -- the cell's state, Diag and
-//    right-hand side, and for each of its neighbour records the neighbour's
-//    state and the face -- and evaluate the neighbour-state half of
-//    FluxLUSGS3D (flux_lusgs_pre), the reciprocal of the diagonal term and
-//    the limiter's velocity square into the team's shared-memory stage slot
-//    (an mbarrier pair per slot hands it over and back);
-//  * consumer warps take an item from its stage into registers, wait at the
-//    level barrier (a named barrier over the consumer warps alone) and run
-//    only the dependent chain: the neighbours' increments, the rest of
-//    FluxLUSGS3D, the ordered sums, the division, the limiter and the stores.
+// Levels are ordered by an mbarrier each (kLevelBars of them in turn): an
+// item arrives when its increments are in the block's ring, and an item waits
+// for the barrier of the level before its own.  A warp's previous item is
+// kSweepWarps items back and every level holds an item, so the level it waits
+// for is less than kSweepWarps levels past the first unfinished one: with
+// kLevelBars >= kSweepWarps the barrier's earlier phases are over, and its
+// next one starts only after the waiting item's own level, so the parity of
+// the phase is never mistaken for another's.
 //
 // A dependency inside the chunk is read from the block's shared-memory ring
 // of its last kRing positions (or, when older, from global memory); a
 // dependency on another chunk is polled in L2 until it is no longer the
-// sentinel (bounded wait).  In the backward sweep the producers also apply
-// the state update of an item's cells (UpdateFlowField3D_CFL3d) once the
-// consumers have released its slot, from the slot's state record and the
-// ring: the update is off the dependent chain and reads nothing twice.  The
-// consumer warps are then at most kWsTeams - 1 items further (a slot is
-// refilled only after every consumer warp has released it), fewer than kRing
-// positions, so the item's ring entries are still there.  Progress: a cell
-// waits only for cells of lower levels, each block visits its levels in
-// increasing order, and every block is resident, so by induction over the
-// levels every cell completes.  Every wait is bounded; one that gives up
-// sets the error word, after which every other wait returns at once and the
-// kernel runs to its end.
+// sentinel (bounded wait).  Both global reads are issued before the level's
+// wait.  The backward sweep applies the state update (UpdateFlowField3D_CFL3d)
+// after the item's arrival, off the dependent chain.  Progress: a cell waits
+// only for cells of lower levels, each warp takes its items in increasing
+// order, and every block is resident, so by induction over the levels every
+// cell completes.  Every wait is bounded; one that gives up sets the error
+// word, after which every other wait returns at once and the kernel runs to
+// its end.
+//
+// What bounds it: the dependent chain of a level -- ring read, product, sum,
+// quotient, limiter, ring write, barrier, about 1100 cycles in a warp alone --
+// times the levels.  Producer warps that stage items in shared memory for
+// lane pairs of other warps (the form before) took 64^3 x 6 cells through the
+// forward / backward sweep in 511 / 565 us, 16^3 x 6 in 117 / 132; this one
+// takes 334 / 396 and 63 / 64.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kMark = 0x80000000u;    // neighbour flag: in another chunk (wait in L2)
 constexpr uint32_t kInRing = 0x40000000u;  // neighbour flag: increment in the block's ring
@@ -1036,7 +1044,16 @@ constexpr int kMinChunk = 64;              // no chunk smaller than this many ce
 constexpr int kRing = MFG_SWEEP_RING;
 static_assert((kRing & (kRing - 1)) == 0, "ring size must be a power of two");
 
-constexpr int kWsTeams = 4;  // producer teams; team t fills stage slot t
+#ifndef MFG_SWEEP_WARPS
+#define MFG_SWEEP_WARPS 12
+#endif
+constexpr int kSweepWarps = MFG_SWEEP_WARPS;
+constexpr int kSweepThreads = 32 * kSweepWarps;
+constexpr int kLevelBars = 16;
+static_assert(kLevelBars >= kSweepWarps, "a waiting warp is less than kLevelBars levels ahead");
+// Arrivals of a level barrier: the first item of a level arrives for all the
+// items the level does not have.
+constexpr uint32_t kLevelArrivals = (1u << 20) - 1;
 // Segment starts of a chunk kept in shared memory (longer chunks read the
 // rest from global memory).
 constexpr int kSegCache = 512;
@@ -1050,22 +1067,12 @@ struct __align__(8) PosCell {
   int32_t cell, ns;
 };
 
-// A cell is swept by a pair of consumer lanes: lane h of the pair owns the
-// records [h W / 2, (h + 1) W / 2), whose products are independent
-// (instruction-level parallelism); lane 0 sums its records into the
-// right-hand side in record order and hands the partial sums to lane 1,
-// which adds its own in order, divides, limits and stores -- the operations
-// and order of the reference's loop, so the same bits.  An item holds
-// kGroups cells: 64 (four consumer warps, one per SM sub-partition) for W =
-// 4, 32 for W = 8, whose stage records are twice the size; a producer
-// thread stages one cell.
+// Lanes per cell (L), records per lane (R) and cells per item of the sweeps.
 template <int W>
-struct WsGeom {
-  static constexpr int kGroups = W == 8 ? 32 : 64;      // cells per item
-  static constexpr int kRh = W / 2;                     // records per consumer lane
-  static constexpr int kConsumers = 2 * kGroups;        // consumer threads
-  static constexpr int kTeamThreads = kGroups;          // producer threads per team
-  static constexpr int kThreads = kConsumers + kWsTeams * kTeamThreads;
+struct SweepGeom {
+  static constexpr int L = W / 2;
+  static constexpr int R = W / L;
+  static constexpr int kCells = 32 / L;
 };
 
 template <bool MX>
@@ -1079,44 +1086,7 @@ struct SweepTypes<true> {
   using Rec = SweepRecF;
 };
 
-// One stage slot: what the producers stage for the cells of one item, each
-// field an array over the item's G cells, so that the consumer warps (one
-// thread per cell) read 32 consecutive words per field without bank
-// conflicts.  A record's fields -- FP64: the neighbour-state half of
-// FluxLUSGS3D (LusgsPre, 11 values), the face normal and the weight;
-// mixed: the neighbour's single-precision state record (8 values), the
-// normal and the weight.  A cell's: its state record, the right-hand side
-// (res, forward; the forward increment, backward), the diagonal term it
-// divides by with its reciprocal, the limiter's velocity square, and the
-// indices.
-template <int W, bool MX>
-struct WsSlot {
-  static constexpr int G = WsGeom<W>::kGroups;
-  static constexpr int kRF = MX ? Q_STRIDE + 4 : 15;
-  typename SweepTypes<MX>::Q rec[W][kRF][G];
-  double qc[Q_STRIDE][G];
-  double in5[5][G];
-  double den[G], rden[G], vv[G];
-  int32_t cell[G], ns[G], first[G], pos[G];
-  uint32_t nb[W][G];
-  int32_t nslot[W][G];
-};
-
-template <int W, bool MX>
-constexpr size_t ws_smem_bytes() {
-  return sizeof(WsSlot<W, MX>) * kWsTeams + sizeof(double) * kRing * 5 +
-         sizeof(int32_t) * (kSegCache + 2) + sizeof(double) * kCaseCache +
-         sizeof(uint64_t) * 2 * kWsTeams;
-}
-// the producers' update reads an item's ring entries up to kWsTeams items on
-static_assert(kWsTeams * WsGeom<4>::kGroups < kRing && kWsTeams * WsGeom<8>::kGroups < kRing,
-              "ring longer than the stage");
-static_assert(sizeof(WsSlot<4, false>) % 16 == 0 && sizeof(WsSlot<8, false>) % 16 == 0 &&
-                  sizeof(WsSlot<4, true>) % 16 == 0 && sizeof(WsSlot<8, true>) % 16 == 0,
-              "slot alignment");
-static_assert(ws_smem_bytes<4, false>() <= 227 * 1024 && ws_smem_bytes<8, false>() <= 227 * 1024 &&
-                  ws_smem_bytes<4, true>() <= 227 * 1024 && ws_smem_bytes<8, true>() <= 227 * 1024,
-              "stage fits in shared memory");
+constexpr int kRingRow = 6;  // doubles of a ring row: five increments and padding to 48 bytes
 
 // Asynchronous copies global -> shared (.cg: from L2, never a stale L1 line).
 __device__ __forceinline__ void cp_async16(void *sdst, const void *gsrc) {
@@ -1135,7 +1105,7 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// mbarrier hand-off between the producer teams and the consumer warps.
+// mbarriers of the sweep levels.
 __device__ __forceinline__ unsigned smem_addr(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }
@@ -1143,10 +1113,11 @@ __device__ __forceinline__ void mbar_init(uint64_t *b, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count)
                : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t *b) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(
-                   smem_addr(b))
-               : "memory");
+__device__ __forceinline__ void mbar_arrive(uint64_t *b, unsigned count) {
+  asm volatile(
+      "{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_addr(b)),
+      "r"(count)
+      : "memory");
 }
 __device__ __forceinline__ bool mbar_test(uint64_t *b, unsigned parity) {
   unsigned ok;
@@ -1160,15 +1131,12 @@ __device__ __forceinline__ bool mbar_test(uint64_t *b, unsigned parity) {
 }
 // Bounded wait for the completion of the phase of the given parity; gives up
 // (setting *err) after `spin` cycles, or soon after another wait gave up.
-// The error word and the clock are read every 64th try only, and a waiter
-// with slack (the producers) sleeps between tries, so that waiting warps
-// take neither issue slots nor L2 requests from the ones that compute.
+// The error word and the clock are read every 64th try only.
 __device__ __forceinline__ void mbar_wait(uint64_t *b, unsigned parity, int *err,
-                                          long long spin, unsigned sleep_ns) {
+                                          long long spin) {
   if (mbar_test(b, parity)) return;
   const long long t0 = clock64();
   for (unsigned tries = 1;; tries++) {
-    if (sleep_ns) __nanosleep(sleep_ns);
     if (mbar_test(b, parity)) return;
     if ((tries & 63) == 0) {
       if (ld_relaxed(err)) return;
@@ -1178,15 +1146,6 @@ __device__ __forceinline__ void mbar_wait(uint64_t *b, unsigned parity, int *err
       }
     }
   }
-}
-// The level barrier of the consumer warps (named barrier 1; the producers
-// never take part).
-template <int N>
-__device__ __forceinline__ void consumers_sync() {
-  if (N > 32)
-    asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory");
-  else
-    __syncwarp();
 }
 
 // Diag of a cell whose dt LimitTimeStep clamps to lim (compute_timestep.cpp
@@ -1214,348 +1173,147 @@ __device__ __forceinline__ double clamp_limit(const Params &P,
   return (dt_max / dt_min > P.ratio_dtmax) ? P.ratio_dtmax * dt_min : -1.0;
 }
 
-// Producer: one item's cells into a stage slot; thread g of the team stages
-// cell g of the item.
-template <int W, bool FWD, bool MX>
-__device__ __forceinline__ void ws_produce(
-    WsSlot<W, MX> &S, int32_t g, int32_t p0, int32_t pend, const PosCell *__restrict__ pcs,
-    const typename SweepTypes<MX>::Rec *__restrict__ prec, const int32_t *__restrict__ pnb,
-    const int32_t *__restrict__ pslot, const double *__restrict__ q8,
-    const typename SweepTypes<MX>::Q *__restrict__ qnb, const double *__restrict__ res,
-    const double *__restrict__ dqf_own, int32_t C, const double *__restrict__ diag,
-    int32_t first_cell, const Params &P0, const Cases &cs) {
-  const int32_t p = p0 + g;
-  if (p >= pend) {
-    S.cell[g] = -1;
-    return;
-  }
-  const PosCell x = pcs[p];
-  const Params P = params_of(P0, cs, x.cell);
-  // the records' indices, then the states, then the products (the padding
-  // slots past ns are not read)
-  uint32_t e[W];
-  int32_t sl[W];
-  typename SweepTypes<MX>::Rec rc[W];
+// An item's indices, read one turn ahead: the position's cell (-1: none) and
+// record count, and the lane's neighbours (flags kMark / kInRing) with their
+// ring slots.
+template <int R>
+struct SweepIdx {
+  int32_t p, cell, ns;
+  uint32_t nb[R];
+  int32_t slot[R];
+};
+
+// What a lane keeps of one of its records: FP64, the neighbour-state half of
+// FluxLUSGS3D, the seed of its reciprocal, the normal out of the cell and the
+// weight; mixed, the neighbour's single-precision state, the normal and the
+// weight.
+template <bool MX>
+struct LaneRec {
+  LusgsPre<double> a;
+  double nx, ny, nz, w;
+  int seed;
+};
+template <>
+struct LaneRec<true> {
+  float q[Q_STRIDE];
+  float nx, ny, nz, w;
+};
+
+// The parameters the dependent chain reads.
+struct ChainP {
+  double gamm1, rho_min, rho_max, p_min, p_max;
+};
+
+// w_j * FluxLUSGS3D(q[nb_j], DQ[nb_j], n_j) of one record; ok is cleared
+// where the divisions have to be taken.  A record the cell does not have holds
+// zeros, with density 1, and gives +0.
+__device__ __forceinline__ void lane_product(const LaneRec<false> &r, const double *DQ,
+                                             const FluxP<double> &P, double *wf, bool &ok) {
+  double f[5];
+  bool okr;
+  flux_lusgs_fin_near(r.a, r.seed, DQ, r.nx, r.ny, r.nz, P, f, okr);
+  ok = ok && okr;
 #pragma unroll
-  for (int j = 0; j < W; j++) {
+  for (int k = 0; k < 5; k++) wf[k] = r.w * f[k];
+}
+// Mixed: the off-diagonal product in FP32, widened.
+__device__ __forceinline__ void lane_product(const LaneRec<true> &r, const double *DQ,
+                                             const FluxP<float> &P, double *wf, bool &) {
+  float df[5], ff[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) df[k] = (float)DQ[k];
+  flux_lusgs_diff(r.q, df, r.nx, r.ny, r.nz, P, ff);
+#pragma unroll
+  for (int k = 0; k < 5; k++) wf[k] = (double)(r.w * ff[k]);
+}
+
+// A cell's increment by one lane, from its tables again, with the divisions
+// themselves and the whole limiter: what an item takes where an operand left
+// the fast forms' windows or the limiter acts.  The neighbours' increments
+// are all there.  Out of line: almost no item comes here.
+struct ExactArgs {
+  double in5[5], qc[5], d[5];
+  Params P;
+};
+template <int W, bool FWD, bool MX>
+__device__ __noinline__ void exact_cell(int32_t p, int32_t ns, const uint32_t *pnb,
+                                        const int32_t *pslot,
+                                        const typename SweepTypes<MX>::Rec *prec,
+                                        const typename SweepTypes<MX>::Q *qnb, const double *src,
+                                        const double *ring, double den, bool limited,
+                                        ExactArgs &t) {
+  double s[5];
+  for (int k = 0; k < 5; k++) s[k] = FWD ? t.in5[k] : 0.0;
+#pragma unroll 1
+  for (int32_t j = 0; j < ns; j++) {
     const int64_t o = (int64_t)p * W + j;
-    if (j >= x.ns) continue;
-    e[j] = (uint32_t)pnb[o];
-    sl[j] = pslot[o];
-    rc[j] = prec[o];
-  }
-  {
-    double qc[Q_STRIDE];
-    load_q(q8, x.cell, qc);
-    const double dg = diag[x.cell];
-    double in5[5];
-#pragma unroll
-    for (int k = 0; k < 5; k++)
-      in5[k] = FWD ? res[(int64_t)k * C + x.cell] : dqf_own[(int64_t)x.cell * Q_STRIDE + k];
-    const double den = FWD ? dg : 2.0 * dg;
-#pragma unroll
-    for (int k = 0; k < Q_STRIDE; k++) S.qc[k][g] = qc[k];
-#pragma unroll
-    for (int k = 0; k < 5; k++) S.in5[k][g] = in5[k];
-    S.den[g] = den;
-    S.rden[g] = 1.0 / den;
-    S.vv[g] = qc[1] * qc[1] + qc[2] * qc[2] + qc[3] * qc[3];
-    S.cell[g] = x.cell;
-    S.ns[g] = x.ns;
-    S.first[g] = FWD && x.cell == (cs.P ? cs.first[case_of(cs, x.cell)] : first_cell);
-    S.pos[g] = p;
-  }
-#pragma unroll
-  for (int j = 0; j < W; j++) {
-    if (j >= x.ns) continue;
-    S.nb[j][g] = e[j];
-    S.nslot[j][g] = sl[j];
-    const int64_t nb = (int64_t)(e[j] & kIdMask);
+    const uint32_t e = pnb[o];
+    const int64_t nb = (int64_t)(e & kIdMask);
+    double dn[5], wf[5];
+    if (e & kInRing)
+      for (int k = 0; k < 5; k++) dn[k] = ring[pslot[o] * kRingRow + k];
+    else
+      load_rec5_l2(src + nb * Q_STRIDE, dn);
+    const typename SweepTypes<MX>::Rec r = prec[o];
     if constexpr (MX) {
-      const float4 *qs = reinterpret_cast<const float4 *>(qnb + nb * Q_STRIDE);
-      const float4 a = __ldg(qs), b = __ldg(qs + 1);
-      const float v[Q_STRIDE] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int k = 0; k < Q_STRIDE; k++) S.rec[j][k][g] = v[k];
-      S.rec[j][Q_STRIDE][g] = rc[j].nx;
-      S.rec[j][Q_STRIDE + 1][g] = rc[j].ny;
-      S.rec[j][Q_STRIDE + 2][g] = rc[j].nz;
-      S.rec[j][Q_STRIDE + 3][g] = rc[j].w;
+      float q[Q_STRIDE], df[5], ff[5];
+      load_q4(qnb, nb, q);
+      for (int k = 0; k < 5; k++) df[k] = (float)dn[k];
+      flux_lusgs_diff(q, df, r.nx, r.ny, r.nz, flux_params<float>(t.P), ff);
+      for (int k = 0; k < 5; k++) wf[k] = (double)(r.w * ff[k]);
     } else {
-      double qn[Q_STRIDE];
-      load_q(qnb, nb, qn);
-      const LusgsPre<double> a =
-          flux_lusgs_pre(qn, rc[j].nx, rc[j].ny, rc[j].nz, flux_params<double>(P));
-      const double v[15] = {a.Q0, a.Q1, a.Q2, a.Q3, a.Q4, a.vq, a.eig, a.f1,
-                            a.f2, a.f3, a.f4, rc[j].nx, rc[j].ny, rc[j].nz, rc[j].w};
-#pragma unroll
-      for (int k = 0; k < 15; k++) S.rec[j][k][g] = v[k];
+      double q[Q_STRIDE], f[5];
+      load_q(qnb, nb, q);
+      flux_lusgs(q, dn, r.nx, r.ny, r.nz, t.P, f);
+      for (int k = 0; k < 5; k++) wf[k] = r.w * f[k];
     }
+    for (int k = 0; k < 5; k++) s[k] = FWD ? s[k] - wf[k] : s[k] + wf[k];
   }
+  for (int k = 0; k < 5; k++) t.d[k] = FWD ? s[k] / den : t.in5[k] - s[k] / den;
+  if (limited) dq_limit(t.qc, t.d, t.P);
 }
 
-// Consumer: the dependent chain of one cell on its lane pair (lane h, see
-// WsGeom), c < 0 when the pair has no cell in this item.  e[u]: the
-// neighbour word of the lane's record u, dn[u]: its increment as read when
-// the item was taken (unless it is in the ring).  FWD: DQ* = (res - sum_j
-// 0.5 area_j F_j) / Diag, limited except for the first cell (SolveLUSGS3D
-// forward, forward_lusgs.cpp:803-1014); backward: DQ = DQ* - (sum_j area_j
-// F_j) / (2 Diag), limited (:1060-1249).
-template <int W, bool FWD, bool MX>
-__device__ __forceinline__ void ws_cell(
-    const WsSlot<W, MX> &S, int32_t g, int32_t h, int32_t c, int32_t ns, const uint32_t *e,
-    double (*dn)[5], int32_t pbase, double *ring, const double *src, double *dst,
-    double *rearm, const Params &P0, const double *s_lim, int clamp_check,
-    double *__restrict__ dt, double *__restrict__ diag,
-    const unsigned long long *__restrict__ dt_ext, const int32_t *__restrict__ cptr,
-    const SlotRec *__restrict__ slots, const double *__restrict__ vol, int *err, long long spin,
-    const Cases &cs) {
-  constexpr int R = WsGeom<W>::kRh;
-  const bool live = c >= 0;
-  // the neighbour increments: from the ring, else as read when the item was
-  // taken, polled again in L2 while one is the sentinel.  The warp polls in
-  // one converged, bounded loop.
-  bool have[R];
-#pragma unroll
-  for (int u = 0; u < R; u++) {
-    const int j = h * R + u;
-    have[u] = true;
-    if (!live || j >= ns) continue;
-    if (e[u] & kInRing) {
-      const int32_t sl = S.nslot[j][g];
-#pragma unroll
-      for (int k = 0; k < 5; k++) dn[u][k] = ring[sl * 5 + k];
-    } else {
-      have[u] = rec5_ready(dn[u]);
-    }
-  }
-  bool all = true;
-#pragma unroll
-  for (int u = 0; u < R; u++) all = all && have[u];
-  if (__any_sync(0xffffffffu, !all)) {
-    const long long t0 = clock64();
-    for (int polls = 1;; polls++) {
-      if (polls > 64) __nanosleep(64);
-      if (!all) {
-        const int gave_up = ld_relaxed(err);
-        all = true;
-#pragma unroll
-        for (int u = 0; u < R; u++) {
-          if (have[u]) continue;
-          load_rec5_l2(src + (int64_t)(e[u] & kIdMask) * Q_STRIDE, dn[u]);
-          have[u] = rec5_ready(dn[u]);
-          all = all && have[u];
-        }
-        if (!all && (gave_up || clock64() - t0 > spin)) {
-          if (!gave_up) atomicExch(err, 1);
-          all = true;  // results invalid; the host reports MFG_ERR_TIMEOUT
-        }
-      }
-      if (!__any_sync(0xffffffffu, !all)) break;
-    }
-  }
-  const int32_t cse = live ? case_of(cs, c) : 0;
-  const Params P = live ? params_of(P0, cs, c) : P0;
-  // w_j * FluxLUSGS3D(q[nb_j], DQ[nb_j], n_j) of the lane's records, their
-  // products overlapping (FP64: branch-free divisions, the exact form redone
-  // for the lane's records when one is out of its window)
-  double wf[R][5];
-  if constexpr (!MX) {
-    auto pre_of = [&](int j) {
-      LusgsPre<double> a;
-      a.Q0 = S.rec[j][0][g];
-      a.Q1 = S.rec[j][1][g];
-      a.Q2 = S.rec[j][2][g];
-      a.Q3 = S.rec[j][3][g];
-      a.Q4 = S.rec[j][4][g];
-      a.vq = S.rec[j][5][g];
-      a.eig = S.rec[j][6][g];
-      a.f1 = S.rec[j][7][g];
-      a.f2 = S.rec[j][8][g];
-      a.f3 = S.rec[j][9][g];
-      a.f4 = S.rec[j][10][g];
-      return a;
-    };
-    bool ok = true;
-#pragma unroll
-    for (int u = 0; u < R; u++) {
-      const int j = h * R + u;
-      if (!live || j >= ns) continue;
-      double f[5];
-      bool oku;
-      flux_lusgs_fin_fast(pre_of(j), dn[u], S.rec[j][11][g], S.rec[j][12][g], S.rec[j][13][g],
-                          flux_params<double>(P), f, oku);
-      ok = ok && oku;
-      const double w = S.rec[j][14][g];
-#pragma unroll
-      for (int k = 0; k < 5; k++) wf[u][k] = w * f[k];
-    }
-    if (!ok) {
-#pragma unroll
-      for (int u = 0; u < R; u++) {
-        const int j = h * R + u;
-        if (!live || j >= ns) continue;
-        double f[5];
-        flux_lusgs_fin(pre_of(j), dn[u], S.rec[j][11][g], S.rec[j][12][g], S.rec[j][13][g],
-                       flux_params<double>(P), f);
-        const double w = S.rec[j][14][g];
-#pragma unroll
-        for (int k = 0; k < 5; k++) wf[u][k] = w * f[k];
-      }
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < R; u++) {
-      const int j = h * R + u;
-      if (!live || j >= ns) continue;
-      // off-diagonal product in FP32, accumulated in FP64
-      float qf[Q_STRIDE], df[5], ff[5];
-#pragma unroll
-      for (int k = 0; k < Q_STRIDE; k++) qf[k] = S.rec[j][k][g];
-#pragma unroll
-      for (int k = 0; k < 5; k++) df[k] = (float)dn[u][k];
-      flux_lusgs_diff(qf, df, S.rec[j][Q_STRIDE][g], S.rec[j][Q_STRIDE + 1][g],
-                      S.rec[j][Q_STRIDE + 2][g], flux_params<float>(P), ff);
-      const float w = S.rec[j][Q_STRIDE + 3][g];
-#pragma unroll
-      for (int k = 0; k < 5; k++) wf[u][k] = (double)(w * ff[k]);
-    }
-  }
-  // the sum over the records in record order: lane 0 from the right-hand
-  // side through its records, lane 1 on from lane 0's partial sums
-  double part[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) part[k] = (FWD && h == 0 && live) ? S.in5[k][g] : 0.0;
-#pragma unroll
-  for (int u = 0; u < R; u++) {
-    const int j = h * R + u;
-    if (!live || j >= ns || h != 0) continue;
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-      if (FWD)
-        part[k] -= wf[u][k];
-      else
-        part[k] += wf[u][k];
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 5; k++) part[k] = __shfl_sync(0xffffffffu, part[k], threadIdx.x & ~1);
-#pragma unroll
-  for (int u = 0; u < R; u++) {
-    const int j = h * R + u;
-    if (!live || j >= ns || h != 1) continue;
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-      if (FWD)
-        part[k] -= wf[u][k];
-      else
-        part[k] += wf[u][k];
-    }
-  }
-  if (!live || h != 1) return;
-  double qc[Q_STRIDE];
-#pragma unroll
-  for (int k = 0; k < Q_STRIDE; k++) qc[k] = S.qc[k][g];
-  const double den = S.den[g], rden = S.rden[g];
-  // LimitTimeStep's clamp (forward sweep of a fused iteration, only when some
-  // case's dt ratio exceeds its limit)
-  double dg = den, lim = -1.0;  // forward: den is Diag itself
-  bool clamped = false;
-  if (FWD && clamp_check) {
-    lim = (cse < kCaseCache) ? s_lim[cse] : clamp_limit(P, dt_ext + 2 * cse);
-    if (lim > 0.0 && dt[c] > lim) {
-      dg = clamped_diag(c, qc, P, lim, cptr, slots, vol);
-      clamped = true;
-    }
-  }
-  // the five quotients overlapping (branch-free; div_by_recip for all when
-  // one of them is out of its window)
-  double d[5];
-  bool okq = true;
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    bool okk;
-    const double qk = div_recip_fast(part[k], den, rden, okk);
-    okq = okq && okk;
-    d[k] = FWD ? qk : S.in5[k][g] - qk;
-  }
-  if (!okq)
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-      const double qk = div_by_recip(part[k], den, rden);
-      d[k] = FWD ? qk : S.in5[k][g] - qk;
-    }
-  if (FWD && clamped)
-#pragma unroll
-    for (int k = 0; k < 5; k++) d[k] = part[k] / dg;
-  if (!FWD || !S.first[g]) dq_limit_vv(qc, S.vv[g], d, P);
-  if (FWD && clamped) {
-    dt[c] = lim;
-    diag[c] = dg;
-  }
-  store_dq(dst, c, d);
-  store_sentinel(rearm, c);  // armed for the other sweep
-  const int32_t slot = (S.pos[g] - pbase) & (kRing - 1);
-#pragma unroll
-  for (int k = 0; k < 5; k++) ring[slot * 5 + k] = d[k];
+// Dynamic shared memory of a sweep: the ring, and per warp the products of
+// its cells' records that lanes other than the first hold.
+template <int W>
+constexpr size_t sweep_smem_bytes() {
+  return sizeof(double) * kRingRow *
+         (kRing + (size_t)kSweepWarps * SweepGeom<W>::kCells * (W - SweepGeom<W>::R));
 }
 
-// Backward sweep, producer thread g: UpdateFlowField3D_CFL3d of cell g of the
-// item whose slot the consumers have just released, from the slot's state
-// record and the cell's final increment in the ring (forward_lusgs.cpp:
-// 1335-1488); the new state goes to the other state buffer.
-template <int W, bool MX>
-__device__ __forceinline__ void ws_update(const WsSlot<W, MX> &S, int32_t g, int32_t pbase,
-                                          const double *ring, double *__restrict__ q8_new,
-                                          float *__restrict__ q4_new, const Params &P0,
-                                          const Cases &cs) {
-  const int32_t c = S.cell[g];
-  if (c < 0) return;
-  double qc[Q_STRIDE], d[5];
-#pragma unroll
-  for (int k = 0; k < Q_STRIDE; k++) qc[k] = S.qc[k][g];
-  const int32_t sl = (S.pos[g] - pbase) & (kRing - 1);
-#pragma unroll
-  for (int k = 0; k < 5; k++) d[k] = ring[sl * 5 + k];
-  const Params P = params_of(P0, cs, c);
-  update_cell(qc, d, P);
-  cell_props(qc, P);
-  store_q(q8_new, c, qc);
-  if (MX) store_q4(q4_new, c, qc);
-}
-
-// One persistent sweep over chunk blockIdx.x (see the section comment).
-template <int W, bool FWD, bool MX>
-__device__ __forceinline__ void ws_sweep(
+// One persistent sweep over chunk blockIdx.x (see the section comment).  FWD:
+// DQ* = (res - sum_j 0.5 area_j F_j) / Diag, limited except for the first
+// cell (SolveLUSGS3D forward, forward_lusgs.cpp:803-1014); backward: DQ = DQ*
+// - (sum_j area_j F_j) / (2 Diag), limited (:1060-1249), then the update.
+template <int W, bool FWD, bool MX, bool BATCH>
+__device__ __forceinline__ void chunk_sweep(
     const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
     const PosCell *__restrict__ pcs, const typename SweepTypes<MX>::Rec *__restrict__ prec,
     const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
     const double *__restrict__ q8, const typename SweepTypes<MX>::Q *__restrict__ qnb,
     const double *src, double *dst, double *rearm, const double *__restrict__ res,
-    const double *__restrict__ dqf_own, int32_t C, double *__restrict__ diag, int32_t first_cell,
-    const Params &P0, int clamp_check, double *__restrict__ dt,
-    const unsigned long long *__restrict__ dt_ext, const int32_t *__restrict__ cptr,
-    const SlotRec *__restrict__ slots, const double *__restrict__ vol, int *err, long long spin,
-    const Cases &cs, double *__restrict__ q8_new, float *__restrict__ q4_new) {
-  using Geo = WsGeom<W>;
-  constexpr int G = Geo::kGroups;
-  extern __shared__ __align__(16) unsigned char ws_smem[];
-  WsSlot<W, MX> *stage = reinterpret_cast<WsSlot<W, MX> *>(ws_smem);  // [kWsTeams]
-  double *ring = reinterpret_cast<double *>(stage + kWsTeams);         // [kRing][5]
-  int32_t *s_segs = reinterpret_cast<int32_t *>(ring + kRing * 5);       // [kSegCache + 1]
-  double *s_lim = reinterpret_cast<double *>(s_segs + kSegCache + 2);    // [kCaseCache]
-  uint64_t *full = reinterpret_cast<uint64_t *>(s_lim + kCaseCache);     // [kWsTeams]
-  uint64_t *empty = full + kWsTeams;                                      // [kWsTeams]
+    const double *dqf_own, int32_t C, double *diag, int32_t first_cell, const Params &P0,
+    int clamp_check, double *dt, const unsigned long long *__restrict__ dt_ext,
+    const int32_t *__restrict__ cptr, const SlotRec *__restrict__ slots,
+    const double *__restrict__ vol, int *err, long long spin, const Cases &cs,
+    double *__restrict__ q8_new, float *__restrict__ q4_new) {
+  using Geo = SweepGeom<W>;
+  constexpr int L = Geo::L, R = Geo::R, kCells = Geo::kCells;
+  extern __shared__ __align__(16) double ring[];  // [kRing][kRingRow]
+  // [kCells][(L - 1) R][kRingRow] of this warp: record u of lane h > 0 of a
+  // cell in row u (L - 1) + h - 1
+  constexpr int kXRows = (L - 1) * R;
+  double *xprod = ring + kRing * kRingRow + (threadIdx.x >> 5) * (kCells * kXRows * kRingRow);
+  __shared__ int32_t s_segs[kSegCache + 1];
+  __shared__ double s_lim[FWD ? kCaseCache : 1];
+  __shared__ uint64_t lbar[kLevelBars];
   __shared__ int s_clamp_any;
   const int32_t sg0 = seg_begin[blockIdx.x], sg1 = seg_begin[blockIdx.x + 1];
   for (int32_t i = threadIdx.x; i <= sg1 - sg0 && i <= kSegCache; i += blockDim.x)
     s_segs[i] = segs[sg0 + i];
   if (threadIdx.x == 0) {
     s_clamp_any = 0;
-    for (int t = 0; t < kWsTeams; t++) {
-      mbar_init(&full[t], Geo::kTeamThreads);
-      mbar_init(&empty[t], Geo::kConsumers / 32);
-    }
+    for (int t = 0; t < kLevelBars; t++) mbar_init(&lbar[t], kLevelArrivals);
   }
   __syncthreads();
   if (FWD && clamp_check)
@@ -1568,103 +1326,306 @@ __device__ __forceinline__ void ws_sweep(
   // the per-cell clamp test only when some case needs it
   clamp_check = (FWD && clamp_check && s_clamp_any) ? 1 : 0;
   const int32_t pbase = sg1 > sg0 ? s_segs[0] : 0;
-  auto seg_at = [&](int32_t sg) {
-    const int32_t i = sg - sg0;
-    return i <= kSegCache ? s_segs[i] : segs[sg];
-  };
-  if (threadIdx.x >= Geo::kConsumers) {
-    // producer team t: items t, t + kWsTeams, ... into stage slot t
-    const int32_t t = (threadIdx.x - Geo::kConsumers) / Geo::kTeamThreads;
-    const int32_t r = (threadIdx.x - Geo::kConsumers) % Geo::kTeamThreads;
-    WsSlot<W, MX> &S = stage[t];
-    int32_t item = 0, last_use = -1;
-    for (int32_t sg = sg0; sg < sg1; sg++) {
-      const int32_t a = seg_at(sg), b = seg_at(sg + 1);
-      const int32_t np = (b - a + G - 1) / G;
-      for (int32_t pass = 0; pass < np; pass++, item++) {
-        if (item % kWsTeams != t) continue;
-        const int32_t use = item / kWsTeams;
-        if (use >= 1) {
-          mbar_wait(&empty[t], (unsigned)((use - 1) & 1), err, spin, 256);
-          if (!FWD) ws_update<W, MX>(S, r, pbase, ring, q8_new, q4_new, P0, cs);
-        }
-        ws_produce<W, FWD, MX>(S, r, a + pass * G, b, pcs, prec, pnb, pslot, q8, qnb, res,
-                               dqf_own, C, diag, first_cell, P0, cs);
-        mbar_arrive(&full[t]);
-        last_use = use;
-      }
-    }
-    if (!FWD && last_use >= 0) {  // the slot's last item
-      mbar_wait(&empty[t], (unsigned)(last_use & 1), err, spin, 256);
-      ws_update<W, MX>(S, r, pbase, ring, q8_new, q4_new, P0, cs);
-    }
-    return;
+  const int32_t lane = threadIdx.x & 31, h = lane & (L - 1), g = lane / L;
+
+  // the item cursor: the next item of this warp and its level's segment
+  // [ca, cb), whose items are [cbase, cbase + cnp)
+  int32_t item = threadIdx.x >> 5, csg = sg0, ca = pbase, cb = pbase, cbase = 0, cnp = 0;
+  if (sg1 > sg0) {
+    cb = 1 <= kSegCache ? s_segs[1] : segs[sg0 + 1];
+    cnp = (cb - ca + kCells - 1) / kCells;
   }
-  // consumers: lane pair g takes cell g of every item
-  constexpr int R = Geo::kRh;
-  const int32_t g = threadIdx.x >> 1, h = threadIdx.x & 1;
-  int32_t item = 0;
-  for (int32_t sg = sg0; sg < sg1; sg++) {
-    const int32_t a = seg_at(sg), b = seg_at(sg + 1);
-    const int32_t np = (b - a + G - 1) / G;
-    for (int32_t pass = 0; pass < np; pass++, item++) {
-      const int32_t t = item % kWsTeams;
-      mbar_wait(&full[t], (unsigned)((item / kWsTeams) & 1), err, spin, 0);
-      const WsSlot<W, MX> &S = stage[t];
-      const int32_t c = S.cell[g];
-      const int32_t ns = c >= 0 ? S.ns[g] : 0;
-      uint32_t e[R];
-      double dn[R][5];
-      // increments read from L2 (older than the ring, or produced by another
-      // chunk) are requested now, so that their round trips overlap the
-      // level barrier; one still holding the sentinel is polled in ws_cell
+  auto seek = [&]() {
+    while (csg < sg1 && item >= cbase + cnp) {
+      cbase += cnp;
+      ++csg;
+      if (csg >= sg1) break;
+      ca = cb;
+      const int32_t i = csg + 1 - sg0;
+      cb = i <= kSegCache ? s_segs[i] : segs[csg + 1];
+      cnp = (cb - ca + kCells - 1) / kCells;
+    }
+  };
+  auto fetch = [&](SweepIdx<R> &o) {
+    o.cell = -1;
+    o.ns = 0;
+    o.p = ca + (item - cbase) * kCells + g;
 #pragma unroll
-      for (int u = 0; u < R; u++) {
-        const int j = h * R + u;
-        e[u] = j < ns ? S.nb[j][g] : kInRing;
-        if (!(e[u] & kInRing)) load_rec5_l2(src + (int64_t)(e[u] & kIdMask) * Q_STRIDE, dn[u]);
+    for (int u = 0; u < R; u++) {
+      o.nb[u] = 0;
+      o.slot[u] = 0;
+    }
+    if (csg >= sg1 || o.p >= cb) return;
+    const PosCell x = pcs[o.p];
+    o.cell = x.cell;
+    o.ns = x.ns;
+#pragma unroll
+    for (int u = 0; u < R; u++) {  // padding reads 0
+      o.nb[u] = (uint32_t)pnb[(int64_t)o.p * W + u * L + h];
+      o.slot[u] = pslot[(int64_t)o.p * W + u * L + h];
+    }
+  };
+  SweepIdx<R> nx;
+  seek();
+  fetch(nx);
+  while (csg < sg1) {
+    const SweepIdx<R> x = nx;
+    const int32_t sg = csg - sg0;  // the item's level within the chunk
+    const unsigned arrivals = item == cbase ? kLevelArrivals - (unsigned)cnp + 1u : 1u;
+    const bool live = x.cell >= 0;
+    const int32_t c = x.cell;
+    const int32_t cse = BATCH && live ? cs.of[c] : 0;
+    const Params *Pc = BATCH ? cs.P + cse : nullptr;
+    // the read-only data of the item
+    double qc[Q_STRIDE], in5[5], den = 1.0;
+    LaneRec<MX> rec[R];
+    FluxP<typename SweepTypes<MX>::Q> FP;
+    if (BATCH)
+      FP = flux_params<typename SweepTypes<MX>::Q>(*Pc);
+    else
+      FP = flux_params<typename SweepTypes<MX>::Q>(P0);
+    ChainP CP;
+    if (BATCH)
+      CP = ChainP{Pc->gamm1, Pc->rho_min, Pc->rho_max, Pc->p_min, Pc->p_max};
+    else
+      CP = ChainP{P0.gamm1, P0.rho_min, P0.rho_max, P0.p_min, P0.p_max};
+    // (a lane without a cell or a record reads its own or the first row, so
+    // that all loads of the item are in flight together)
+    const int32_t cl = live ? c : 0, pl = live ? x.p : 0;
+    bool has[R];
+    typename SweepTypes<MX>::Q qn[R][Q_STRIDE];
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      has[u] = u * L + h < x.ns;
+      const int64_t nb = has[u] ? (int64_t)(x.nb[u] & kIdMask) : (int64_t)cl;
+      const typename SweepTypes<MX>::Rec *rp = prec + (int64_t)pl * W + u * L + h;
+      if constexpr (MX) {
+        const float4 f = __ldg(reinterpret_cast<const float4 *>(rp));
+        rec[u].nx = f.x; rec[u].ny = f.y; rec[u].nz = f.z; rec[u].w = f.w;
+        ldg_v8f(qnb + nb * Q_STRIDE, qn[u]);
+      } else {
+        ldg_v4(&rp->nx, rec[u].nx, rec[u].ny, rec[u].nz, rec[u].w);
+        load_q_w(qnb, nb, qn[u]);
       }
-      if (pass == 0 && item > 0) consumers_sync<Geo::kConsumers>();  // the previous level is stored
-      ws_cell<W, FWD, MX>(S, g, h, c, ns, e, dn, pbase, ring, src, dst, rearm, P0, s_lim,
-                          clamp_check,
-                          dt, diag, dt_ext, cptr, slots, vol, err, spin, cs);
+    }
+    load_q_w(q8, cl, qc);
+    const double dg = diag[cl];
+    if (FWD) {
+#pragma unroll
+      for (int k = 0; k < 5; k++) in5[k] = __ldg(res + (int64_t)k * C + cl);
+    } else {
+      const double2 *pp = reinterpret_cast<const double2 *>(dqf_own + (int64_t)cl * Q_STRIDE);
+      const double2 a = pp[0], b = pp[1];
+      in5[0] = a.x; in5[1] = a.y; in5[2] = b.x; in5[3] = b.y;
+      in5[4] = dqf_own[(int64_t)cl * Q_STRIDE + 4];
+    }
+    // the next item's indices
+    item += kSweepWarps;
+    seek();
+    fetch(nx);
+    double dn[R][5];
+    bool have[R];
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      have[u] = true;
+#pragma unroll
+      for (int k = 0; k < 5; k++) dn[u][k] = 0.0;
+      // a record the cell does not have: zeros, density 1
+      if constexpr (MX) {
+#pragma unroll
+        for (int k = 0; k < Q_STRIDE; k++) rec[u].q[k] = has[u] ? qn[u][k] : (k == 0 ? 1.0f : 0.0f);
+        if (!has[u]) rec[u].nx = rec[u].ny = rec[u].nz = rec[u].w = 0.0f;
+      } else {
+        rec[u].a = flux_lusgs_pre(qn[u], rec[u].nx, rec[u].ny, rec[u].nz, FP);
+        rec[u].seed = rcp_seed(qn[u][0]);
+        if (!has[u]) {
+          rec[u] = LaneRec<MX>{};
+          rec[u].a.Q0 = 1.0;
+          rec[u].seed = __double2hiint(1.0);
+        }
+      }
+    }
+    // LimitTimeStep's clamp (forward sweep of a fused iteration, only when
+    // some case's dt ratio exceeds its limit)
+    den = FWD ? dg : 2.0 * dg;
+    double lim = -1.0;
+    if (FWD && clamp_check && live) {
+      const Params &P = BATCH ? *Pc : P0;
+      lim = (cse < kCaseCache) ? s_lim[cse] : clamp_limit(P, dt_ext + 2 * cse);
+      if (lim > 0.0 && dt[c] > lim)
+        den = clamped_diag(c, qc, P, lim, cptr, slots, vol);
+      else
+        lim = -1.0;
+    }
+    const double rden = 1.0 / den;
+    const double vv = qc[1] * qc[1] + qc[2] * qc[2] + qc[3] * qc[3];
+    const bool limited = !FWD || c != (BATCH && live ? cs.first[cse] : first_cell);
+    const bool second = __any_sync(0xffffffffu, x.ns > L);  // some lane has two records
+    // increments read from L2 (older than the ring, or produced by another
+    // chunk), polled while one is the sentinel: the warp polls in one
+    // converged, bounded loop, before the level's wait
+    bool l2 = false;
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      have[u] = !has[u] || (x.nb[u] & kInRing);
+      l2 = l2 || !have[u];
+    }
+    if (__any_sync(0xffffffffu, l2)) {
+      const long long t0 = clock64();
+      for (int polls = 1;; polls++) {
+        if (polls > 64) __nanosleep(64);
+        bool all = true;
+        if (l2) {
+          const int gave_up = ld_relaxed(err);
+#pragma unroll
+          for (int u = 0; u < R; u++) {
+            if (have[u]) continue;
+            load_rec5_l2(src + (int64_t)(x.nb[u] & kIdMask) * Q_STRIDE, dn[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < R; u++) {
+            if (!have[u]) have[u] = rec5_ready(dn[u]);
+            all = all && have[u];
+          }
+          l2 = !all;
+          if (!all && (gave_up || clock64() - t0 > spin)) {
+            if (!gave_up) atomicExch(err, 1);
+            all = true;  // results invalid; the host reports MFG_ERR_TIMEOUT
+          }
+        }
+        if (!__any_sync(0xffffffffu, !all)) break;
+      }
+    }
+    // the level before this one is in the ring
+    if (sg > 0)
+      mbar_wait(&lbar[(sg - 1) % kLevelBars], (unsigned)((sg - 1) / kLevelBars) & 1u, err, spin);
+#pragma unroll
+    for (int u = 0; u < R; u++)
+      if (has[u] && (x.nb[u] & kInRing)) {
+        const double2 *rr = reinterpret_cast<const double2 *>(ring + x.slot[u] * kRingRow);
+        const double2 a = rr[0], b = rr[1];
+        dn[u][0] = a.x; dn[u][1] = a.y; dn[u][2] = b.x; dn[u][3] = b.y;
+        dn[u][4] = ring[x.slot[u] * kRingRow + 4];
+      }
+    // the dependent chain: the lanes' products, handed to the cell's first
+    // lane, which sums them in record order (the other lanes go through the
+    // motions), divides and tests the limiter
+    double s[5], d[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) s[k] = FWD ? in5[k] : 0.0;
+    bool ok = true;
+    auto chain = [&](auto NN) {
+      constexpr int N = decltype(NN)::value;
+      double wf[N][5];
+#pragma unroll
+      for (int u = 0; u < N; u++) lane_product(rec[u], dn[u], FP, wf[u], ok);
+      double2 *mine = reinterpret_cast<double2 *>(xprod + (g * kXRows + h - 1) * kRingRow);
+      const double2 *theirs = reinterpret_cast<const double2 *>(xprod + g * kXRows * kRingRow);
+      if (h > 0) {
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+          double2 *row = mine + u * (L - 1) * (kRingRow / 2);
+          row[0] = make_double2(wf[u][0], wf[u][1]);
+          row[1] = make_double2(wf[u][2], wf[u][3]);
+          row[2] = make_double2(wf[u][4], 0.0);
+        }
+      }
       __syncwarp();
-      if ((threadIdx.x & 31) == 0) mbar_arrive(&empty[t]);  // the slot is free again
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) s[k] = FWD ? s[k] - wf[u][k] : s[k] + wf[u][k];
+#pragma unroll
+        for (int hh = 1; hh < L; hh++) {
+          const double2 *row = theirs + (u * (L - 1) + hh - 1) * (kRingRow / 2);
+          const double2 a = row[0], b = row[1];
+          const double v[5] = {a.x, a.y, b.x, b.y, row[2].x};
+#pragma unroll
+          for (int k = 0; k < 5; k++) s[k] = FWD ? s[k] - v[k] : s[k] + v[k];
+        }
+      }
+    };
+    if (second)
+      chain(std::integral_constant<int, R>());
+    else
+      chain(std::integral_constant<int, 1>());
+    bool okd = true;
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      bool okk;
+      const double qk = div_recip_zero(s[k], den, rden, okk);
+      okd = okd && okk;
+      d[k] = FWD ? qk : in5[k] - qk;
+    }
+    const bool redo = h == 0 && live && (!okd || (limited && dq_over_limit(qc, vv, d, CP)));
+    if (__any_sync(0xffffffffu, redo || !ok) && h == 0 && live) {
+      ExactArgs t;  // copies, so that the arrays above stay in registers
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        t.in5[k] = in5[k];
+        t.qc[k] = qc[k];
+      }
+      t.P = BATCH ? *Pc : P0;
+      exact_cell<W, FWD, MX>(x.p, x.ns, reinterpret_cast<const uint32_t *>(pnb), pslot, prec, qnb,
+                             src, ring, den, limited, t);
+#pragma unroll
+      for (int k = 0; k < 5; k++) d[k] = t.d[k];
+    }
+    if (h == 0 && live) {
+      double2 *rr =
+          reinterpret_cast<double2 *>(ring + ((x.p - pbase) & (kRing - 1)) * kRingRow);
+      rr[0] = make_double2(d[0], d[1]);
+      rr[1] = make_double2(d[2], d[3]);
+      rr[2] = make_double2(d[4], 0.0);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&lbar[sg % kLevelBars], arrivals);
+    // off the chain: the increment for the other chunks, the other sweep's
+    // sentinel, and in the backward sweep the state update
+    if (live && h == 0) {
+      store_dq(dst, c, d);
+      store_sentinel(rearm, c);  // armed for the other sweep
+      if (FWD && lim > 0.0) {
+        dt[c] = lim;
+        diag[c] = den;
+      }
+      if (!FWD) {
+        const Params &P = BATCH ? *Pc : P0;
+        update_cell(qc, d, P);
+        cell_props(qc, P);
+        store_q(q8_new, c, qc);
+        if (MX) store_q4(q4_new, c, qc);
+      }
     }
   }
 }
 
-#ifndef MFG_PERSIST_MINB
-#define MFG_PERSIST_MINB 1
-#endif
-
 // Forward sweep.  chunk_skip > 0 withholds the first chunk_skip chunks
 // (failure-detection self-test only: the cells that depend on them wait
 // until the bound runs out).
-template <int W, bool MX>
-__global__ void __launch_bounds__(WsGeom<W>::kThreads, MFG_PERSIST_MINB)
+template <int W, bool MX, bool BATCH>
+__global__ void __launch_bounds__(kSweepThreads, 1)
 k_sweep_fwd_chunk(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
                   const PosCell *__restrict__ pcs,
                   const typename SweepTypes<MX>::Rec *__restrict__ prec,
                   const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
                   const double *__restrict__ q8,
                   const typename SweepTypes<MX>::Q *__restrict__ qnb, double *dqf,
-                  double *__restrict__ dqb, const double *__restrict__ res, int32_t C,
-                  double *__restrict__ diag, int32_t first_cell, Params P0, int clamp_check,
-                  double *__restrict__ dt, const unsigned long long *__restrict__ dt_ext,
+                  double *dqb, const double *__restrict__ res, int32_t C,
+                  double *diag, int32_t first_cell, Params P0, int clamp_check,
+                  double *dt, const unsigned long long *__restrict__ dt_ext,
                   const int32_t *__restrict__ cptr, const SlotRec *__restrict__ slots,
                   const double *__restrict__ vol, int *err, long long spin,
                   int32_t chunk_skip, Cases cs) {
   if ((int32_t)blockIdx.x < chunk_skip) return;
-  ws_sweep<W, true, MX>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqf, dqf, dqb, res,
-                        nullptr, C, diag, first_cell, P0, clamp_check, dt, dt_ext, cptr, slots,
-                        vol, err, spin, cs, nullptr, nullptr);
+  chunk_sweep<W, true, MX, BATCH>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqf, dqf, dqb,
+                                  res, nullptr, C, diag, first_cell, P0, clamp_check, dt, dt_ext,
+                                  cptr, slots, vol, err, spin, cs, nullptr, nullptr);
 }
 
-// Backward sweep with the state update (by the producers, see the section
-// comment).
-template <int W, bool MX>
-__global__ void __launch_bounds__(WsGeom<W>::kThreads, MFG_PERSIST_MINB)
+// Backward sweep with the state update (see the section comment).
+template <int W, bool MX, bool BATCH>
+__global__ void __launch_bounds__(kSweepThreads, 1)
 k_sweep_bwd_chunk(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
                   const PosCell *__restrict__ pcs,
                   const typename SweepTypes<MX>::Rec *__restrict__ prec,
@@ -1672,11 +1633,12 @@ k_sweep_bwd_chunk(const int32_t *__restrict__ seg_begin, const int32_t *__restri
                   const double *__restrict__ q8,
                   const typename SweepTypes<MX>::Q *__restrict__ qnb,
                   double *__restrict__ q8_new, float *__restrict__ q4_new,
-                  double *__restrict__ dqf, double *dqb, const double *__restrict__ diag,
+                  double *dqf, double *dqb, const double *__restrict__ diag,
                   Params P0, int *err, long long spin, Cases cs) {
-  ws_sweep<W, false, MX>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqb, dqb, dqf, nullptr,
-                         dqf, 0, const_cast<double *>(diag), 0, P0, 0, nullptr, nullptr, nullptr,
-                         nullptr, nullptr, err, spin, cs, q8_new, q4_new);
+  chunk_sweep<W, false, MX, BATCH>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqb, dqb, dqf,
+                                   nullptr, dqf, 0, const_cast<double *>(diag), 0, P0, 0, nullptr,
+                                   nullptr, nullptr, nullptr, nullptr, err, spin, cs, q8_new,
+                                   q4_new);
 }
 
 // ---------------------------------------------------------------------------
@@ -2748,7 +2710,8 @@ __global__ void k_selftest_functions(int mode, int32_t n, Params P, const double
     const FluxP<double> fp = flux_params<double>(P);
     const LusgsPre<double> a = flux_lusgs_pre(q, c[10], c[11], c[12], fp);
     bool ok = false;
-    if (mode == 3) flux_lusgs_fin_fast(a, dq, c[10], c[11], c[12], fp, f, ok);
+    if (mode == 3)
+      flux_lusgs_fin_near(a, rcp_seed(q[0]), dq, c[10], c[11], c[12], fp, f, ok);
     if (!ok) flux_lusgs_fin(a, dq, c[10], c[11], c[12], fp, f);
     for (int k = 0; k < 5; k++) out[5 * (int64_t)i + k] = f[k];
   } else {
@@ -2796,6 +2759,20 @@ __global__ void k_selftest_division_fast(int64_t n, uint64_t seed,
     bool okq;
     const double q = div_recip_fast(a, b, y, okq);
     if (okq && __double_as_longlong(q) != __double_as_longlong(a / b)) b1++;
+    // from the seed of a divisor within 1/16 of b
+    const double b0f = b * (1.0 + ((double)(int64_t)(ra >> 12) * 0x1p-52 - 0.5) * 0.115);
+    double near;
+    bool okn;
+    const double yn = rcp_rn_near(b, __hiloint2double(rcp_seed(b0f), 0), near, okn);
+    if (!okn) {
+      if (fabs(b) > 0x1p-119 && fabs(b) < 0x1p119) b0++;  // inside the window
+    } else {
+      if (__double_as_longlong(yn) != __double_as_longlong(1.0 / b)) b0++;
+      const double qn = div_recip_near(a, b, near, yn, okq);
+      if (okq && __double_as_longlong(qn) != __double_as_longlong(a / b)) b1++;
+      const double z = div_recip_near(0.0, b, near, yn, okq);
+      if (!okq || __double_as_longlong(z) != __double_as_longlong(0.0 / b)) b1++;
+    }
   }
   if (b0) atomicAdd(bad, b0);
   if (b1) atomicAdd(bad + 1, b1);
@@ -2944,41 +2921,38 @@ __global__ void k_halo_nodes_mx(int32_t nu, const int32_t *__restrict__ unodes,
 // context
 // ---------------------------------------------------------------------------
 
-// The persistent sweep kernel for (W, precision) and its dynamic shared
-// memory.
-// kind MFG_SWEEP_DEEP: the warp-specialised kernels (one block per SM);
-// MFG_SWEEP_WIDE: the many-block kernels for wide levels.
-static const void *sweep_kernel(bool fwd, int w, bool mx, int kind = MFG_SWEEP_DEEP) {
-#define MFG_SK(W_)                                                                           \
-  if (w == W_ && kind == MFG_SWEEP_DEEP)                                                     \
-    return fwd ? (mx ? (const void *)k_sweep_fwd_chunk<W_, true>                               \
-                     : (const void *)k_sweep_fwd_chunk<W_, false>)                             \
-               : (mx ? (const void *)k_sweep_bwd_chunk<W_, true>                               \
-                     : (const void *)k_sweep_bwd_chunk<W_, false>);                            \
-  if (w == W_ && kind == MFG_SWEEP_WIDE)                                                     \
-    return fwd ? (mx ? (const void *)k_sweep_fwd_wide<W_, W_, true>                            \
-                     : (const void *)k_sweep_fwd_wide<W_, W_, false>)                          \
-               : (mx ? (const void *)k_sweep_bwd_wide<W_, W_, true>                            \
-                     : (const void *)k_sweep_bwd_wide<W_, W_, false>);
-  MFG_SK(4)
-  MFG_SK(8)
+// The persistent sweep kernel for (W, precision, one grid or a batch).
+// kind MFG_SWEEP_DEEP: one block per SM; MFG_SWEEP_WIDE: the many-block
+// kernels for wide levels.
+static const void *sweep_kernel(bool fwd, int w, bool mx, bool batch, int kind = MFG_SWEEP_DEEP) {
+#define MFG_SK(W_, MX_)                                                                     \
+  if (w == W_ && mx == MX_ && kind == MFG_SWEEP_DEEP)                                        \
+    return fwd ? (batch ? (const void *)k_sweep_fwd_chunk<W_, MX_, true>                      \
+                        : (const void *)k_sweep_fwd_chunk<W_, MX_, false>)                    \
+               : (batch ? (const void *)k_sweep_bwd_chunk<W_, MX_, true>                      \
+                        : (const void *)k_sweep_bwd_chunk<W_, MX_, false>);                   \
+  if (w == W_ && mx == MX_ && kind == MFG_SWEEP_WIDE)                                        \
+    return fwd ? (const void *)k_sweep_fwd_wide<W_, W_, MX_>                                  \
+               : (const void *)k_sweep_bwd_wide<W_, W_, MX_>;
+  MFG_SK(4, false)
+  MFG_SK(4, true)
+  MFG_SK(8, false)
+  MFG_SK(8, true)
 #undef MFG_SK
   return nullptr;
 }
-static int sweep_threads(int w, int kind = MFG_SWEEP_DEEP) {
-  if (kind == MFG_SWEEP_WIDE) return kWideBlock;
-  return w == 8 ? WsGeom<8>::kThreads : WsGeom<4>::kThreads;
+static int sweep_threads(int kind) {
+  return kind == MFG_SWEEP_WIDE ? kWideBlock : kSweepThreads;
 }
-static size_t sweep_smem(int w, bool mx, int kind = MFG_SWEEP_DEEP) {
+static size_t sweep_smem(int w, int kind) {
   if (kind == MFG_SWEEP_WIDE) return 0;
-  if (w == 8) return mx ? ws_smem_bytes<8, true>() : ws_smem_bytes<8, false>();
-  return mx ? ws_smem_bytes<4, true>() : ws_smem_bytes<4, false>();
+  return w == 8 ? sweep_smem_bytes<8>() : sweep_smem_bytes<4>();
 }
-// Cells per work item (lane groups of a block) and ring positions of a
-// kernel kind.
+// Cells of a level that a kernel kind's block sweeps side by side (as the
+// chunk model counts them), and the ring positions of a kind.
 static int32_t sweep_groups(int w, int kind = MFG_SWEEP_DEEP) {
   if (kind == MFG_SWEEP_WIDE) return kWideBlock / std::max(w, 1);
-  return w == 8 ? WsGeom<8>::kGroups : WsGeom<4>::kGroups;
+  return w == 8 ? 32 : 64;
 }
 static int32_t sweep_ring(int kind) { return kind == MFG_SWEEP_WIDE ? kWideRing : kRing; }
 
@@ -4245,22 +4219,21 @@ static int ctx_begin(int32_t n_node, int32_t n_face, int32_t n_cell, int32_t n_b
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     // resident blocks per SM of each kernel pair (both sweeps), with the
-    // stage's dynamic shared memory allowed first
+    // sweeps' dynamic shared memory allowed first
     const bool mx = precision == MFG_PREC_MIXED;
     for (int kind = 0; kind < 2; kind++)
       for (int wi = 0; wi < 2; wi++) {
-        const int w = wi ? 8 : 4;
         int per_sm = 1 << 30;
         for (bool fwd : {true, false}) {
-          const void *fn = sweep_kernel(fwd, w, mx, kind);
-          const size_t smem = sweep_smem(w, mx, kind);
+          const void *fn = sweep_kernel(fwd, wi ? 8 : 4, mx, cl.ncase > 1, kind);
+          const size_t smem = sweep_smem(wi ? 8 : 4, kind);
           if (smem &&
               cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
                   cudaSuccess)
             return fail(MFG_ERR_CUDA);
           int b = 0;
-          if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, sweep_threads(w, kind),
-                                                            smem) != cudaSuccess)
+          if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, sweep_threads(kind), smem) !=
+              cudaSuccess)
             return fail(MFG_ERR_CUDA);
           per_sm = std::min(per_sm, b);
         }
@@ -5406,10 +5379,10 @@ static int launch_fwd_persist(mfg_ctx *ctx, bool clamp_check, int32_t chunk_skip
                   (void *)&qnb, &ctx->dqf, &ctx->dq8, &ctx->res, &C, &ctx->diag, &first, &P,
                   &clamp, &ctx->dt, &ctx->dt_ext, &ctx->cptr, &ctx->slots, &ctx->vol,
                   &ctx->sweep_err, &spin, &skip, &cs};
-  const void *fn = sweep_kernel(true, ctx->sweep_w, mx, ctx->sweep_kind);
+  const void *fn = sweep_kernel(true, ctx->sweep_w, mx, ctx->ncase > 1, ctx->sweep_kind);
   if (!fn) return MFG_ERR_UNSUPPORTED;
-  return launch_coop(fn, ctx->nchunks, sweep_threads(ctx->sweep_w, ctx->sweep_kind),
-                     sweep_smem(ctx->sweep_w, mx, ctx->sweep_kind), ctx->stream, args);
+  return launch_coop(fn, ctx->nchunks, sweep_threads(ctx->sweep_kind),
+                     sweep_smem(ctx->sweep_w, ctx->sweep_kind), ctx->stream, args);
 }
 
 static int launch_bwd_persist(mfg_ctx *ctx, long long spin) {
@@ -5425,10 +5398,11 @@ static int launch_bwd_persist(mfg_ctx *ctx, long long spin) {
   void *args[] = {&w.seg_begin, &w.segs, &w.cells, &recs, &w.nbs, &w.nslots, (void *)&q,
                   (void *)&qnb, &qn, &q4n, &ctx->dqf, &ctx->dq8, &ctx->diag, &P,
                   &ctx->sweep_err, &spin, &cs};
-  const void *fn = sweep_kernel(false, ctx->sweep_w, mx, ctx->sweep_kind);
+  const void *fn = sweep_kernel(false, ctx->sweep_w, mx, ctx->ncase > 1, ctx->sweep_kind);
   if (!fn) return MFG_ERR_UNSUPPORTED;
-  const int rc = launch_coop(fn, ctx->nchunks, sweep_threads(ctx->sweep_w, ctx->sweep_kind),
-                             sweep_smem(ctx->sweep_w, mx, ctx->sweep_kind), ctx->stream, args);
+  const int rc =
+      launch_coop(fn, ctx->nchunks, sweep_threads(ctx->sweep_kind),
+                  sweep_smem(ctx->sweep_w, ctx->sweep_kind), ctx->stream, args);
   if (rc || ctx->sweep_kind != MFG_SWEEP_WIDE) return rc;
   // the wide sweeps leave the update to a streaming pass
   if (mx)
