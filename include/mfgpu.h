@@ -218,15 +218,11 @@ int mfg_plan_chunks(int32_t C, int32_t L, const int32_t *lptr, const int32_t *ce
                     const int32_t *sptr, const int32_t *nbs, const double *xc,
                     const double *yc, const double *zc, int32_t P, int32_t G, int32_t force,
                     int32_t *assign, int32_t *grid, double *est_us);
-/* The persistent sweep kernels.  MFG_SWEEP_DEEP: one block per SM, producer
- * warps staging each cell's static terms ahead for consumer lane pairs that
- * run only the dependent chain -- short per-level latency, for levels of up
- * to about 128 cells per SM.  MFG_SWEEP_WIDE: many 64-thread blocks per SM
- * with small chunks -- for wider levels, whose latency one block hides
- * behind another's work.  A context takes WIDE when its widest level would
- * give a DEEP block more than two passes per level; mfg_set_sweep_kernel
- * forces a kind for contexts created afterwards (-1 restores the default).
- * Identical results either way. */
+/* The persistent sweep kernels, in two launch shapes.  MFG_SWEEP_DEEP: one
+ * block of 12 warps and one chunk per SM, the default.  MFG_SWEEP_WIDE: two
+ * blocks of 6 warps and two chunks per SM.  mfg_set_sweep_kernel forces a
+ * kind for contexts created afterwards (-1 restores the default).  Identical
+ * results either way. */
 #define MFG_SWEEP_DEEP 0
 #define MFG_SWEEP_WIDE 1
 int mfg_set_sweep_kernel(int32_t kind);

@@ -988,21 +988,21 @@ k_sweep_bwd(int32_t l0, int32_t l1, const int32_t *__restrict__ cells,
 }
 
 // ---------------------------------------------------------------------------
-// Persistent chunked sweeps, one block per SM.
+// Persistent chunked sweeps.
 //
 // The cells are split into chunks, one per block (cooperative launch).  A
-// chunk's positions are level-major; a level's positions are cut into items
-// of 32 / L cells, and the items of the chunk, in level order, go to the
-// block's warps in turn.  A warp sweeps its item alone: lane h of a cell's L
-// lanes owns the records h, h + L, ... of the cell.  Before its turn it reads
+// chunk's positions are level-major, and within a level cells of many records
+// come first; a level's positions are cut into items of 32 / L cells, and the
+// items of the chunk, in level order, go to the block's warps in turn.  A warp
+// sweeps its item alone: lane h of a cell's L lanes owns the records h, h + L,
+// ... of the cell (most items need one per lane).  Before its turn it reads
 // everything of the item that no sweep writes -- the states of the cells and
 // of their neighbours, the faces, Diag, the right-hand side -- and forms what
 // they give (the neighbour-state half of FluxLUSGS3D, the diagonal term's
-// reciprocal) in registers; the dependent chain then holds only the
-// neighbours' increments, the rest of FluxLUSGS3D, the ordered sums, the
-// quotients and the limiter.  While one warp runs its chain, the others read
-// ahead or store: with kSweepWarps warps and a few items per level, a warp
-// reads several levels ahead of its turn.
+// reciprocal); the dependent chain then holds only the neighbours'
+// increments, the rest of FluxLUSGS3D, the ordered sums, the quotients and the
+// limiter's test.  While one warp runs its chain, the others read ahead or
+// store.
 //
 // Levels are ordered by an mbarrier each (kLevelBars of them in turn): an
 // item arrives when its increments are in the block's ring, and an item waits
@@ -1014,23 +1014,30 @@ k_sweep_bwd(int32_t l0, int32_t l1, const int32_t *__restrict__ cells,
 // the phase is never mistaken for another's.
 //
 // A dependency inside the chunk is read from the block's shared-memory ring
-// of its last kRing positions (or, when older, from global memory); a
-// dependency on another chunk is polled in L2 until it is no longer the
-// sentinel (bounded wait).  Both global reads are issued before the level's
-// wait.  The backward sweep applies the state update (UpdateFlowField3D_CFL3d)
-// after the item's arrival, off the dependent chain.  Progress: a cell waits
-// only for cells of lower levels, each warp takes its items in increasing
-// order, and every block is resident, so by induction over the levels every
-// cell completes.  Every wait is bounded; one that gives up sets the error
-// word, after which every other wait returns at once and the kernel runs to
-// its end.
+// of its last kRing positions.  One in another chunk, or older than the ring,
+// comes from L2: it is copied into a row of the lane's own while the item's
+// other data are read, and polled (bounded) while it is still the sentinel.
+// Only the rows that some record reads from L2 are armed with the sentinel
+// (PosCell's kArm).  Progress: a cell waits only for cells of lower levels,
+// each warp takes its items in increasing order, and every block is resident,
+// so by induction over the levels every cell completes.  Every wait is
+// bounded; one that gives up sets the error word, after which every other wait
+// returns at once and the kernel runs to its end.
 //
 // What bounds it: the dependent chain of a level -- ring read, product, sum,
-// quotient, limiter, ring write, barrier, about 1100 cycles in a warp alone --
-// times the levels.  Producer warps that stage items in shared memory for
-// lane pairs of other warps (the form before) took 64^3 x 6 cells through the
-// forward / backward sweep in 511 / 565 us, 16^3 x 6 in 117 / 132; this one
-// takes 334 / 396 and 63 / 64.
+// quotient, limiter, ring write, barrier, about 900 cycles in a warp alone --
+// and a warp's turn (about 3500 cycles of loads ahead of the chain), shared by
+// kSweepWarps warps; then the L1's data pipe, whose row gathers and stores
+// keep it half busy at 64^3.  Forward / backward sweep, us, the latter with
+// k_update_cells (the forms before: producer warps staging items in shared
+// memory for lane pairs of other warps, update by the producers; then whole
+// items per warp with the update in the sweep, a sentinel for every row, the
+// L2 increments polled before the level's wait and one level search per
+// level): 64^3 x 6 cells 511 / 565, 334 / 396, now 270 / 322; 128^3 3057 /
+// 3157 (blocks of two warps), -, 1758 / 2147; 16^3 117 / 132, 63 / 64, 57 /
+// 62.  Measured and not kept: thread-per-cell items (353 / 429), 14 or 16
+// warps of 128 registers (spills; 362 / 408), the item's rows by cp.async a
+// turn ahead (317 / 375: their shared-memory round trip loads the data pipe).
 // ---------------------------------------------------------------------------
 constexpr uint32_t kMark = 0x80000000u;    // neighbour flag: in another chunk (wait in L2)
 constexpr uint32_t kInRing = 0x40000000u;  // neighbour flag: increment in the block's ring
@@ -1044,11 +1051,8 @@ constexpr int kMinChunk = 64;              // no chunk smaller than this many ce
 constexpr int kRing = MFG_SWEEP_RING;
 static_assert((kRing & (kRing - 1)) == 0, "ring size must be a power of two");
 
-#ifndef MFG_SWEEP_WARPS
-#define MFG_SWEEP_WARPS 12
-#endif
-constexpr int kSweepWarps = MFG_SWEEP_WARPS;
-constexpr int kSweepThreads = 32 * kSweepWarps;
+// Warps per SM, in one block (MFG_SWEEP_DEEP) or two (MFG_SWEEP_WIDE).
+constexpr int kSweepWarps = 12;
 constexpr int kLevelBars = 16;
 static_assert(kLevelBars >= kSweepWarps, "a waiting warp is less than kLevelBars levels ahead");
 // Arrivals of a level barrier: the first item of a level arrives for all the
@@ -1063,8 +1067,16 @@ constexpr int kCaseCache = 128;
 // Position-major sweep tables.  Position p (chunk-major, level-sorted) holds
 // one cell; its records sit at [p * W, p * W + ns).  W = 4 (tetrahedra) or 8
 // (any cell with at most 8 lower or upper neighbours).
+// ns holds the record count, and kArm where the other sweep reads the cell's
+// increment from L2: its row is then armed with the sentinel in this sweep.
 struct __align__(8) PosCell {
   int32_t cell, ns;
+};
+constexpr int kArm = 256;
+// A record's neighbour (flags kMark / kInRing) and, in the ring, its row.
+struct __align__(8) SweepNb {
+  uint32_t nb;
+  int32_t slot;
 };
 
 // Lanes per cell (L), records per lane (R) and cells per item of the sweeps.
@@ -1151,16 +1163,21 @@ __device__ __forceinline__ void mbar_wait(uint64_t *b, unsigned parity, int *err
 // Diag of a cell whose dt LimitTimeStep clamps to lim (compute_timestep.cpp
 // :929-944, then Diag = vol / dt + the face sum of CalDiagLUSGS,
 // forward_lusgs.cpp:96 and :175-260, with that dt).
-__device__ __forceinline__ double clamped_diag(int32_t c, const double *qc, const Params &P,
-                                               double lim, const int32_t *__restrict__ cptr,
-                                               const SlotRec *__restrict__ slots,
-                                               const double *__restrict__ vol) {
+// Out of line: only a clamped run's cells come here.
+__device__ __noinline__ double clamped_diag(int32_t c, const double *__restrict__ q8,
+                                            double lhs_omga, double lim,
+                                            const int32_t *__restrict__ cptr,
+                                            const SlotRec *__restrict__ slots,
+                                            const double *__restrict__ vol) {
+  double qc[Q_STRIDE];
+  load_q(q8, c, qc);
   double dg = vol[c] / lim;
+#pragma unroll 1
   for (int32_t s = cptr[c]; s < cptr[c + 1]; s++) {
     const SlotRec sr = slots[s];
     double vn = qc[1] * sr.nx + qc[2] * sr.ny + qc[3] * sr.nz;
     vn = fabs(vn);
-    dg += 0.5 * sr.area * (vn + qc[Q_A]) * P.lhs_omga;
+    dg += 0.5 * sr.area * (vn + qc[Q_A]) * lhs_omga;
   }
   return dg;
 }
@@ -1173,14 +1190,20 @@ __device__ __forceinline__ double clamp_limit(const Params &P,
   return (dt_max / dt_min > P.ratio_dtmax) ? P.ratio_dtmax * dt_min : -1.0;
 }
 
-// An item's indices, read one turn ahead: the position's cell (-1: none) and
-// record count, and the lane's neighbours (flags kMark / kInRing) with their
-// ring slots.
+// An item of a warp: its level within the chunk (-1: no item) and its arrivals
+// at the level's barrier, whether the lane has a cell, and its position.
+struct SweepItem {
+  int32_t sg;
+  uint32_t arrivals;
+  bool live;
+  int32_t p;
+};
+// The lane's tables at that position, copied into shared memory one turn ahead
+// (registers loaded so early would cost the block a warp or spills).
 template <int R>
 struct SweepIdx {
-  int32_t p, cell, ns;
-  uint32_t nb[R];
-  int32_t slot[R];
+  PosCell x;
+  SweepNb r[R];
 };
 
 // What a lane keeps of one of its records: FP64, the neighbour-state half of
@@ -1204,21 +1227,19 @@ struct ChainP {
   double gamm1, rho_min, rho_max, p_min, p_max;
 };
 
-// w_j * FluxLUSGS3D(q[nb_j], DQ[nb_j], n_j) of one record; ok is cleared
+// w_j * FluxLUSGS3D(q[nb_j], DQ[nb_j], n_j) of one record; bad turns negative
 // where the divisions have to be taken.  A record the cell does not have holds
 // zeros, with density 1, and gives +0.
 __device__ __forceinline__ void lane_product(const LaneRec<false> &r, const double *DQ,
-                                             const FluxP<double> &P, double *wf, bool &ok) {
+                                             const FluxP<double> &P, double *wf, int &bad) {
   double f[5];
-  bool okr;
-  flux_lusgs_fin_near(r.a, r.seed, DQ, r.nx, r.ny, r.nz, P, f, okr);
-  ok = ok && okr;
+  flux_lusgs_fin_near(r.a, r.seed, DQ, r.nx, r.ny, r.nz, P, f, bad);
 #pragma unroll
   for (int k = 0; k < 5; k++) wf[k] = r.w * f[k];
 }
 // Mixed: the off-diagonal product in FP32, widened.
 __device__ __forceinline__ void lane_product(const LaneRec<true> &r, const double *DQ,
-                                             const FluxP<float> &P, double *wf, bool &) {
+                                             const FluxP<float> &P, double *wf, int &) {
   float df[5], ff[5];
 #pragma unroll
   for (int k = 0; k < 5; k++) df[k] = (float)DQ[k];
@@ -1236,8 +1257,7 @@ struct ExactArgs {
   Params P;
 };
 template <int W, bool FWD, bool MX>
-__device__ __noinline__ void exact_cell(int32_t p, int32_t ns, const uint32_t *pnb,
-                                        const int32_t *pslot,
+__device__ __noinline__ void exact_cell(int32_t p, int32_t ns, const SweepNb *pnb,
                                         const typename SweepTypes<MX>::Rec *prec,
                                         const typename SweepTypes<MX>::Q *qnb, const double *src,
                                         const double *ring, double den, bool limited,
@@ -1247,11 +1267,11 @@ __device__ __noinline__ void exact_cell(int32_t p, int32_t ns, const uint32_t *p
 #pragma unroll 1
   for (int32_t j = 0; j < ns; j++) {
     const int64_t o = (int64_t)p * W + j;
-    const uint32_t e = pnb[o];
+    const uint32_t e = pnb[o].nb;
     const int64_t nb = (int64_t)(e & kIdMask);
     double dn[5], wf[5];
     if (e & kInRing)
-      for (int k = 0; k < 5; k++) dn[k] = ring[pslot[o] * kRingRow + k];
+      for (int k = 0; k < 5; k++) dn[k] = ring[pnb[o].slot * kRingRow + k];
     else
       load_rec5_l2(src + nb * Q_STRIDE, dn);
     const typename SweepTypes<MX>::Rec r = prec[o];
@@ -1273,44 +1293,56 @@ __device__ __noinline__ void exact_cell(int32_t p, int32_t ns, const uint32_t *p
   if (limited) dq_limit(t.qc, t.d, t.P);
 }
 
-// Dynamic shared memory of a sweep: the ring, and per warp the products of
-// its cells' records that lanes other than the first hold.
-template <int W>
+// Dynamic shared memory of a sweep: the ring, one row of zeros (the increment
+// of a record a cell does not have), per lane and record a row for an
+// increment read from L2, so that the dependent chain reads every increment
+// from a row of shared memory, and per cell what only its first lane needs,
+// after the products (kOwn units of 16 bytes: the state and the limiter's
+// velocity square, the right-hand side, the divisor and its reciprocal); kept
+// in registers that would cost a quarter of the block's warps.  Then the
+// lanes' indices (SweepIdx).
+constexpr int kOwn = 7;
+template <int W, int NW>
 constexpr size_t sweep_smem_bytes() {
-  return sizeof(double) * kRingRow *
-         (kRing + (size_t)kSweepWarps * SweepGeom<W>::kCells * (W - SweepGeom<W>::R));
+  return sizeof(double) * kRingRow * (kRing + 1 + (size_t)32 * NW * SweepGeom<W>::R) +
+         (size_t)16 * kOwn * SweepGeom<W>::kCells * NW +
+         sizeof(SweepIdx<SweepGeom<W>::R>) * 32 * NW;
 }
 
 // One persistent sweep over chunk blockIdx.x (see the section comment).  FWD:
 // DQ* = (res - sum_j 0.5 area_j F_j) / Diag, limited except for the first
 // cell (SolveLUSGS3D forward, forward_lusgs.cpp:803-1014); backward: DQ = DQ*
 // - (sum_j area_j F_j) / (2 Diag), limited (:1060-1249), then the update.
-template <int W, bool FWD, bool MX, bool BATCH>
+template <int W, bool FWD, bool MX, bool BATCH, int NW>
 __device__ __forceinline__ void chunk_sweep(
     const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
+    const int32_t *__restrict__ seg_items,
     const PosCell *__restrict__ pcs, const typename SweepTypes<MX>::Rec *__restrict__ prec,
-    const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
-    const double *__restrict__ q8, const typename SweepTypes<MX>::Q *__restrict__ qnb,
+    const SweepNb *__restrict__ pnb, const double *__restrict__ q8,
+    const typename SweepTypes<MX>::Q *__restrict__ qnb,
     const double *src, double *dst, double *rearm, const double *__restrict__ res,
     const double *dqf_own, int32_t C, double *diag, int32_t first_cell, const Params &P0,
     int clamp_check, double *dt, const unsigned long long *__restrict__ dt_ext,
     const int32_t *__restrict__ cptr, const SlotRec *__restrict__ slots,
-    const double *__restrict__ vol, int *err, long long spin, const Cases &cs,
-    double *__restrict__ q8_new, float *__restrict__ q4_new) {
+    const double *__restrict__ vol, int *err, long long spin, const Cases &cs) {
   using Geo = SweepGeom<W>;
   constexpr int L = Geo::L, R = Geo::R, kCells = Geo::kCells;
   extern __shared__ __align__(16) double ring[];  // [kRing][kRingRow]
-  // [kCells][(L - 1) R][kRingRow] of this warp: record u of lane h > 0 of a
-  // cell in row u (L - 1) + h - 1
-  constexpr int kXRows = (L - 1) * R;
-  double *xprod = ring + kRing * kRingRow + (threadIdx.x >> 5) * (kCells * kXRows * kRingRow);
-  __shared__ int32_t s_segs[kSegCache + 1];
+  constexpr int kZeroRow = kRing, kL2Row = kRing + 1;
+  // [kOwn][kCells] of this warp
+  double2 *own = reinterpret_cast<double2 *>(ring + (kL2Row + 32 * NW * R) * kRingRow) +
+                 (threadIdx.x >> 5) * (kOwn * kCells);
+  SweepIdx<R> *idx =
+      reinterpret_cast<SweepIdx<R> *>(own + (NW - (threadIdx.x >> 5)) * (kOwn * kCells)) +
+      threadIdx.x;
+  __shared__ int2 s_segs[kSegCache + 1];  // first position and first item
   __shared__ double s_lim[FWD ? kCaseCache : 1];
   __shared__ uint64_t lbar[kLevelBars];
   __shared__ int s_clamp_any;
   const int32_t sg0 = seg_begin[blockIdx.x], sg1 = seg_begin[blockIdx.x + 1];
   for (int32_t i = threadIdx.x; i <= sg1 - sg0 && i <= kSegCache; i += blockDim.x)
-    s_segs[i] = segs[sg0 + i];
+    s_segs[i] = make_int2(segs[sg0 + i], seg_items[sg0 + i]);
+  if (threadIdx.x < kRingRow) ring[kZeroRow * kRingRow + threadIdx.x] = 0.0;
   if (threadIdx.x == 0) {
     s_clamp_any = 0;
     for (int t = 0; t < kLevelBars; t++) mbar_init(&lbar[t], kLevelArrivals);
@@ -1325,691 +1357,305 @@ __device__ __forceinline__ void chunk_sweep(
   __syncthreads();
   // the per-cell clamp test only when some case needs it
   clamp_check = (FWD && clamp_check && s_clamp_any) ? 1 : 0;
-  const int32_t pbase = sg1 > sg0 ? s_segs[0] : 0;
+  const int32_t pbase = sg1 > sg0 ? s_segs[0].x : 0;
   const int32_t lane = threadIdx.x & 31, h = lane & (L - 1), g = lane / L;
 
   // the item cursor: the next item of this warp and its level's segment
-  // [ca, cb), whose items are [cbase, cbase + cnp)
-  int32_t item = threadIdx.x >> 5, csg = sg0, ca = pbase, cb = pbase, cbase = 0, cnp = 0;
-  if (sg1 > sg0) {
-    cb = 1 <= kSegCache ? s_segs[1] : segs[sg0 + 1];
-    cnp = (cb - ca + kCells - 1) / kCells;
-  }
+  // [ca, cb), whose items are [cbase, cbase + cnp).  The warp's lanes look at
+  // the next 32 segments together.
+  int32_t item = (sg1 > sg0 ? s_segs[0].y : 0) + (threadIdx.x >> 5);
+  int32_t csg = sg0, ca = pbase, cb = pbase, cbase = 0, cnp = 0;
+  auto seg_at = [&](int32_t sg) {
+    const int32_t i = sg - sg0;
+    return i <= kSegCache ? s_segs[i] : make_int2(segs[sg], seg_items[sg]);
+  };
   auto seek = [&]() {
-    while (csg < sg1 && item >= cbase + cnp) {
-      cbase += cnp;
-      ++csg;
-      if (csg >= sg1) break;
-      ca = cb;
-      const int32_t i = csg + 1 - sg0;
-      cb = i <= kSegCache ? s_segs[i] : segs[csg + 1];
-      cnp = (cb - ca + kCells - 1) / kCells;
+    while (csg < sg1) {
+      const int32_t sg = csg + 1 + lane;  // where segment csg + lane ends
+      const unsigned past = __ballot_sync(0xffffffffu, sg <= sg1 && item >= seg_at(sg).y);
+      csg += past == 0xffffffffu ? 32 : __ffs(~past) - 1;
+      if (past != 0xffffffffu) break;
     }
+    if (csg >= sg1) return;
+    const int2 a = seg_at(csg), b = seg_at(csg + 1);
+    ca = a.x;
+    cb = b.x;
+    cbase = a.y;
+    cnp = b.y - cbase;
   };
-  auto fetch = [&](SweepIdx<R> &o) {
-    o.cell = -1;
-    o.ns = 0;
-    o.p = ca + (item - cbase) * kCells + g;
+  // the cursor's item, the copy of its indices (a lane without a position reads
+  // the level's last one), and the cursor on to the warp's next
+  auto fetch = [&](SweepItem &o) {
+    seek();
+    o.sg = csg < sg1 ? csg - sg0 : -1;
+    o.arrivals = item == cbase ? kLevelArrivals - (unsigned)cnp + 1u : 1u;
+    const int32_t p = ca + (item - cbase) * kCells + g;
+    o.live = o.sg >= 0 && p < cb;
+    o.p = o.live ? p : max(cb - 1, 0);
+    item += NW;
+    cp_async8(&idx->x, pcs + o.p);
 #pragma unroll
-    for (int u = 0; u < R; u++) {
-      o.nb[u] = 0;
-      o.slot[u] = 0;
-    }
-    if (csg >= sg1 || o.p >= cb) return;
-    const PosCell x = pcs[o.p];
-    o.cell = x.cell;
-    o.ns = x.ns;
-#pragma unroll
-    for (int u = 0; u < R; u++) {  // padding reads 0
-      o.nb[u] = (uint32_t)pnb[(int64_t)o.p * W + u * L + h];
-      o.slot[u] = pslot[(int64_t)o.p * W + u * L + h];
-    }
+    for (int u = 0; u < R; u++)  // padding holds zeros
+      cp_async8(&idx->r[u], pnb + (int64_t)o.p * W + u * L + h);
+    cp_async_commit();
   };
-  SweepIdx<R> nx;
-  seek();
+  SweepItem nx;
   fetch(nx);
-  while (csg < sg1) {
-    const SweepIdx<R> x = nx;
-    const int32_t sg = csg - sg0;  // the item's level within the chunk
-    const unsigned arrivals = item == cbase ? kLevelArrivals - (unsigned)cnp + 1u : 1u;
-    const bool live = x.cell >= 0;
-    const int32_t c = x.cell;
-    const int32_t cse = BATCH && live ? cs.of[c] : 0;
+  while (nx.sg >= 0) {
+    cp_async_wait<0>();
+    const SweepItem x = nx;
+    const int32_t c = idx->x.cell;
+    // the other sweep reads this increment's array from L2: arm its row
+    const bool arm = (idx->x.ns & kArm) != 0;
+    const int32_t ns = x.live ? idx->x.ns & (kArm - 1) : 0;
+    SweepNb rnb[R];
+#pragma unroll
+    for (int u = 0; u < R; u++) rnb[u] = idx->r[u];
+    fetch(nx);
+    const int32_t cse = BATCH ? cs.of[c] : 0;
+    const int32_t sg = x.sg;  // the item's level within the chunk
+    const bool live = x.live;
     const Params *Pc = BATCH ? cs.P + cse : nullptr;
-    // the read-only data of the item
-    double qc[Q_STRIDE], in5[5], den = 1.0;
-    LaneRec<MX> rec[R];
     FluxP<typename SweepTypes<MX>::Q> FP;
     if (BATCH)
       FP = flux_params<typename SweepTypes<MX>::Q>(*Pc);
     else
       FP = flux_params<typename SweepTypes<MX>::Q>(P0);
-    ChainP CP;
-    if (BATCH)
-      CP = ChainP{Pc->gamm1, Pc->rho_min, Pc->rho_max, Pc->p_min, Pc->p_max};
-    else
-      CP = ChainP{P0.gamm1, P0.rho_min, P0.rho_max, P0.p_min, P0.p_max};
-    // (a lane without a cell or a record reads its own or the first row, so
-    // that all loads of the item are in flight together)
-    const int32_t cl = live ? c : 0, pl = live ? x.p : 0;
-    bool has[R];
-    typename SweepTypes<MX>::Q qn[R][Q_STRIDE];
-#pragma unroll
-    for (int u = 0; u < R; u++) {
-      has[u] = u * L + h < x.ns;
-      const int64_t nb = has[u] ? (int64_t)(x.nb[u] & kIdMask) : (int64_t)cl;
-      const typename SweepTypes<MX>::Rec *rp = prec + (int64_t)pl * W + u * L + h;
-      if constexpr (MX) {
-        const float4 f = __ldg(reinterpret_cast<const float4 *>(rp));
-        rec[u].nx = f.x; rec[u].ny = f.y; rec[u].nz = f.z; rec[u].w = f.w;
-        ldg_v8f(qnb + nb * Q_STRIDE, qn[u]);
-      } else {
-        ldg_v4(&rp->nx, rec[u].nx, rec[u].ny, rec[u].nz, rec[u].w);
-        load_q_w(qnb, nb, qn[u]);
-      }
-    }
-    load_q_w(q8, cl, qc);
-    const double dg = diag[cl];
-    if (FWD) {
-#pragma unroll
-      for (int k = 0; k < 5; k++) in5[k] = __ldg(res + (int64_t)k * C + cl);
-    } else {
-      const double2 *pp = reinterpret_cast<const double2 *>(dqf_own + (int64_t)cl * Q_STRIDE);
-      const double2 a = pp[0], b = pp[1];
-      in5[0] = a.x; in5[1] = a.y; in5[2] = b.x; in5[3] = b.y;
-      in5[4] = dqf_own[(int64_t)cl * Q_STRIDE + 4];
-    }
-    // the next item's indices
-    item += kSweepWarps;
-    seek();
-    fetch(nx);
-    double dn[R][5];
-    bool have[R];
-#pragma unroll
-    for (int u = 0; u < R; u++) {
-      have[u] = true;
-#pragma unroll
-      for (int k = 0; k < 5; k++) dn[u][k] = 0.0;
-      // a record the cell does not have: zeros, density 1
-      if constexpr (MX) {
-#pragma unroll
-        for (int k = 0; k < Q_STRIDE; k++) rec[u].q[k] = has[u] ? qn[u][k] : (k == 0 ? 1.0f : 0.0f);
-        if (!has[u]) rec[u].nx = rec[u].ny = rec[u].nz = rec[u].w = 0.0f;
-      } else {
-        rec[u].a = flux_lusgs_pre(qn[u], rec[u].nx, rec[u].ny, rec[u].nz, FP);
-        rec[u].seed = rcp_seed(qn[u][0]);
-        if (!has[u]) {
-          rec[u] = LaneRec<MX>{};
-          rec[u].a.Q0 = 1.0;
-          rec[u].seed = __double2hiint(1.0);
-        }
-      }
-    }
-    // LimitTimeStep's clamp (forward sweep of a fused iteration, only when
-    // some case's dt ratio exceeds its limit)
-    den = FWD ? dg : 2.0 * dg;
-    double lim = -1.0;
-    if (FWD && clamp_check && live) {
-      const Params &P = BATCH ? *Pc : P0;
-      lim = (cse < kCaseCache) ? s_lim[cse] : clamp_limit(P, dt_ext + 2 * cse);
-      if (lim > 0.0 && dt[c] > lim)
-        den = clamped_diag(c, qc, P, lim, cptr, slots, vol);
-      else
-        lim = -1.0;
-    }
-    const double rden = 1.0 / den;
-    const double vv = qc[1] * qc[1] + qc[2] * qc[2] + qc[3] * qc[3];
-    const bool limited = !FWD || c != (BATCH && live ? cs.first[cse] : first_cell);
-    const bool second = __any_sync(0xffffffffu, x.ns > L);  // some lane has two records
-    // increments read from L2 (older than the ring, or produced by another
-    // chunk), polled while one is the sentinel: the warp polls in one
-    // converged, bounded loop, before the level's wait
-    bool l2 = false;
-#pragma unroll
-    for (int u = 0; u < R; u++) {
-      have[u] = !has[u] || (x.nb[u] & kInRing);
-      l2 = l2 || !have[u];
-    }
-    if (__any_sync(0xffffffffu, l2)) {
-      const long long t0 = clock64();
-      for (int polls = 1;; polls++) {
-        if (polls > 64) __nanosleep(64);
-        bool all = true;
-        if (l2) {
-          const int gave_up = ld_relaxed(err);
-#pragma unroll
-          for (int u = 0; u < R; u++) {
-            if (have[u]) continue;
-            load_rec5_l2(src + (int64_t)(x.nb[u] & kIdMask) * Q_STRIDE, dn[u]);
-          }
-#pragma unroll
-          for (int u = 0; u < R; u++) {
-            if (!have[u]) have[u] = rec5_ready(dn[u]);
-            all = all && have[u];
-          }
-          l2 = !all;
-          if (!all && (gave_up || clock64() - t0 > spin)) {
-            if (!gave_up) atomicExch(err, 1);
-            all = true;  // results invalid; the host reports MFG_ERR_TIMEOUT
-          }
-        }
-        if (!__any_sync(0xffffffffu, !all)) break;
-      }
-    }
-    // the level before this one is in the ring
-    if (sg > 0)
-      mbar_wait(&lbar[(sg - 1) % kLevelBars], (unsigned)((sg - 1) / kLevelBars) & 1u, err, spin);
-#pragma unroll
-    for (int u = 0; u < R; u++)
-      if (has[u] && (x.nb[u] & kInRing)) {
-        const double2 *rr = reinterpret_cast<const double2 *>(ring + x.slot[u] * kRingRow);
-        const double2 a = rr[0], b = rr[1];
-        dn[u][0] = a.x; dn[u][1] = a.y; dn[u][2] = b.x; dn[u][3] = b.y;
-        dn[u][4] = ring[x.slot[u] * kRingRow + 4];
-      }
-    // the dependent chain: the lanes' products, handed to the cell's first
-    // lane, which sums them in record order (the other lanes go through the
-    // motions), divides and tests the limiter
-    double s[5], d[5];
-#pragma unroll
-    for (int k = 0; k < 5; k++) s[k] = FWD ? in5[k] : 0.0;
-    bool ok = true;
-    auto chain = [&](auto NN) {
+    // the read-only data of the item; a lane without a record reads its
+    // cell's row instead, so that all loads are in flight together
+    // one turn, with up to N records per lane
+    auto turn = [&](auto NN) {
       constexpr int N = decltype(NN)::value;
-      double wf[N][5];
-#pragma unroll
-      for (int u = 0; u < N; u++) lane_product(rec[u], dn[u], FP, wf[u], ok);
-      double2 *mine = reinterpret_cast<double2 *>(xprod + (g * kXRows + h - 1) * kRingRow);
-      const double2 *theirs = reinterpret_cast<const double2 *>(xprod + g * kXRows * kRingRow);
-      if (h > 0) {
-#pragma unroll
-        for (int u = 0; u < N; u++) {
-          double2 *row = mine + u * (L - 1) * (kRingRow / 2);
-          row[0] = make_double2(wf[u][0], wf[u][1]);
-          row[1] = make_double2(wf[u][2], wf[u][3]);
-          row[2] = make_double2(wf[u][4], 0.0);
+      LaneRec<MX> rec[N];
+      bool has[N], far[N];
+      typename SweepTypes<MX>::Q qn[N][Q_STRIDE];
+      auto load_rec = [&](int u) {
+        has[u] = u * L + h < ns;
+        const int64_t nb = has[u] ? (int64_t)(rnb[u].nb & kIdMask) : (int64_t)c;
+        const typename SweepTypes<MX>::Rec *rp = prec + (int64_t)x.p * W + u * L + h;
+        if constexpr (MX) {
+          const float4 f = __ldg(reinterpret_cast<const float4 *>(rp));
+          rec[u].nx = f.x; rec[u].ny = f.y; rec[u].nz = f.z; rec[u].w = f.w;
+          ldg_v8f(qnb + nb * Q_STRIDE, qn[u]);
+        } else {
+          ldg_v4(&rp->nx, rec[u].nx, rec[u].ny, rec[u].nz, rec[u].w);
+          load_q_w(qnb, nb, qn[u]);
         }
-      }
-      __syncwarp();
+      };
+      auto form_rec = [&](int u) {
+        // a record the cell does not have: zeros, density 1
+        if constexpr (MX) {
+#pragma unroll
+          for (int k = 0; k < Q_STRIDE; k++) rec[u].q[k] = has[u] ? qn[u][k] : (k == 0 ? 1.0f : 0.0f);
+          if (!has[u]) rec[u].nx = rec[u].ny = rec[u].nz = rec[u].w = 0.0f;
+        } else {
+          rec[u].a = flux_lusgs_pre(qn[u], rec[u].nx, rec[u].ny, rec[u].nz, FP);
+          rec[u].seed = rcp_seed(qn[u][0]);
+          if (!has[u]) {
+            rec[u] = LaneRec<MX>{};
+            rec[u].a.Q0 = 1.0;
+            rec[u].seed = __double2hiint(1.0);
+          }
+        }
+      };
+#pragma unroll
+      for (int u = 0; u < N; u++) load_rec(u);
+      // increments that come from L2 (older than the ring, or another chunk's):
+      // copied into the lane's rows while the rest is read and formed
+      int row[N];
+      bool l2 = false;
 #pragma unroll
       for (int u = 0; u < N; u++) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) s[k] = FWD ? s[k] - wf[u][k] : s[k] + wf[u][k];
-#pragma unroll
-        for (int hh = 1; hh < L; hh++) {
-          const double2 *row = theirs + (u * (L - 1) + hh - 1) * (kRingRow / 2);
-          const double2 a = row[0], b = row[1];
-          const double v[5] = {a.x, a.y, b.x, b.y, row[2].x};
-#pragma unroll
-          for (int k = 0; k < 5; k++) s[k] = FWD ? s[k] - v[k] : s[k] + v[k];
+        const bool in_ring = (rnb[u].nb & kInRing) != 0;
+        far[u] = has[u] && !in_ring;
+        l2 = l2 || far[u];
+        row[u] = !has[u] ? kZeroRow : in_ring ? rnb[u].slot : kL2Row + (int)threadIdx.x * R + u;
+        if (far[u]) {
+          const double *rec5 = src + (int64_t)(rnb[u].nb & kIdMask) * Q_STRIDE;
+          double *to = ring + row[u] * kRingRow;
+          cp_async16(to, rec5);
+          cp_async16(to + 2, rec5 + 2);
+          cp_async16(to + 4, rec5 + 4);
         }
       }
-    };
-    if (second)
-      chain(std::integral_constant<int, R>());
-    else
-      chain(std::integral_constant<int, 1>());
-    bool okd = true;
+      if (l2) cp_async_commit();
+      {
+        double qc[Q_STRIDE], in5[5];
+        load_q5_w(q8, c, qc);
+        const double dg = diag[c];
+        if (FWD) {
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
-      bool okk;
-      const double qk = div_recip_zero(s[k], den, rden, okk);
-      okd = okd && okk;
-      d[k] = FWD ? qk : in5[k] - qk;
-    }
-    const bool redo = h == 0 && live && (!okd || (limited && dq_over_limit(qc, vv, d, CP)));
-    if (__any_sync(0xffffffffu, redo || !ok) && h == 0 && live) {
-      ExactArgs t;  // copies, so that the arrays above stay in registers
+          for (int k = 0; k < 5; k++) in5[k] = __ldg(res + (int64_t)k * C + c);
+        } else {
+          const double2 *pp = reinterpret_cast<const double2 *>(dqf_own + (int64_t)c * Q_STRIDE);
+          const double2 a = pp[0], b = pp[1];
+          in5[0] = a.x; in5[1] = a.y; in5[2] = b.x; in5[3] = b.y;
+          in5[4] = dqf_own[(int64_t)c * Q_STRIDE + 4];
+        }
+        // LimitTimeStep's clamp (forward sweep of a fused iteration, only when
+        // some case's dt ratio exceeds its limit)
+        double den = FWD ? dg : 2.0 * dg;
+        if (FWD && clamp_check) {
+          if (live && h == 0) {
+            const Params &P = BATCH ? *Pc : P0;
+            const double lim = (cse < kCaseCache) ? s_lim[cse] : clamp_limit(P, dt_ext + 2 * cse);
+            if (lim > 0.0 && dt[c] > lim) {
+              den = clamped_diag(c, q8, P.lhs_omga, lim, cptr, slots, vol);
+              dt[c] = lim;
+              diag[c] = den;
+            }
+          }
+        }
+        const double rden = 1.0 / den;
+        const double vv = qc[1] * qc[1] + qc[2] * qc[2] + qc[3] * qc[3];
+        if (h == 0) {
+          own[g] = make_double2(qc[0], qc[1]);
+          own[kCells + g] = make_double2(qc[2], qc[3]);
+          own[2 * kCells + g] = make_double2(qc[4], vv);
+          own[3 * kCells + g] = make_double2(in5[0], in5[1]);
+          own[4 * kCells + g] = make_double2(in5[2], in5[3]);
+          own[5 * kCells + g] = make_double2(in5[4], 0.0);
+          own[6 * kCells + g] = make_double2(den, rden);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < N; u++) form_rec(u);
+      // the forward sweep's first cell is not limited
+      const int limits = !FWD || c != (BATCH && live ? cs.first[cse] : first_cell) ? -1 : 0;
+      // the increments from L2 have come; one that was not yet written is polled
+      // until it is (the warp in one converged, bounded loop)
+      if (l2) {
+        cp_async_wait<0>();
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+          if (!far[u]) continue;
+          const double2 *rr = reinterpret_cast<const double2 *>(ring + row[u] * kRingRow);
+          const double2 a = rr[0], b = rr[1];
+          const double dn[5] = {a.x, a.y, b.x, b.y, rr[2].x};
+          far[u] = !rec5_ready(dn);
+        }
+      }
+      bool all = true;
+#pragma unroll
+      for (int u = 0; u < N; u++) all = all && !far[u];
+      if (__any_sync(0xffffffffu, !all)) {
+        const long long t0 = clock64();
+        for (int polls = 1;; polls++) {
+          if (polls > 64) __nanosleep(64);
+          if (!all) {
+            const int gave_up = ld_relaxed(err);
+            double dn[N][5];
+#pragma unroll
+            for (int u = 0; u < N; u++)
+              if (far[u]) load_rec5_l2(src + (int64_t)(rnb[u].nb & kIdMask) * Q_STRIDE, dn[u]);
+            all = true;
+#pragma unroll
+            for (int u = 0; u < N; u++) {
+              if (!far[u]) continue;
+              far[u] = !rec5_ready(dn[u]);
+              all = all && !far[u];
+              double2 *to = reinterpret_cast<double2 *>(ring + row[u] * kRingRow);
+              to[0] = make_double2(dn[u][0], dn[u][1]);
+              to[1] = make_double2(dn[u][2], dn[u][3]);
+              to[2] = make_double2(dn[u][4], 0.0);
+            }
+            if (!all && (gave_up || clock64() - t0 > spin)) {
+              if (!gave_up) atomicExch(err, 1);
+              all = true;  // results invalid; the host reports MFG_ERR_TIMEOUT
+            }
+          }
+          if (!__any_sync(0xffffffffu, !all)) break;
+        }
+      }
+      // the level before this one is in the ring
+      if (sg > 0)
+        mbar_wait(&lbar[(sg - 1) % kLevelBars], (unsigned)((sg - 1) / kLevelBars) & 1u, err, spin);
+      // the dependent chain: the lanes' products, handed to the cell's first
+      // lane, which sums them in record order (the other lanes go through the
+      // motions), divides and tests the limiter
+      double s[5], d[5], in5[5];
+      int bad = 0;
+      double wf[N][5];
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+        const double2 *rr = reinterpret_cast<const double2 *>(ring + row[u] * kRingRow);
+        const double2 a = rr[0], b = rr[1];
+        const double dn[5] = {a.x, a.y, b.x, b.y, rr[2].x};
+        lane_product(rec[u], dn, FP, wf[u], bad);
+      }
+      {
+        const double2 a = own[3 * kCells + g], b = own[4 * kCells + g];
+        in5[0] = a.x; in5[1] = a.y; in5[2] = b.x; in5[3] = b.y;
+        in5[4] = own[5 * kCells + g].x;
+      }
+#pragma unroll
+      for (int k = 0; k < 5; k++) s[k] = FWD ? in5[k] : 0.0;
+#pragma unroll
+      for (int u = 0; u < N; u++)
+#pragma unroll
+        for (int hh = 0; hh < L; hh++)
+#pragma unroll
+          for (int k = 0; k < 5; k++) {
+            const double v = hh ? __shfl_down_sync(0xffffffffu, wf[u][k], hh, L) : wf[u][k];
+            s[k] = FWD ? s[k] - v : s[k] + v;
+          }
+      ChainP CP;
+      if (BATCH)
+        CP = ChainP{Pc->gamm1, Pc->rho_min, Pc->rho_max, Pc->p_min, Pc->p_max};
+      else
+        CP = ChainP{P0.gamm1, P0.rho_min, P0.rho_max, P0.p_min, P0.p_max};
+      const double2 dd = own[6 * kCells + g];
+      const double den = dd.x, rden = dd.y;
+      int badc = outside_exp(den, 523, 1523);
 #pragma unroll
       for (int k = 0; k < 5; k++) {
-        t.in5[k] = in5[k];
-        t.qc[k] = qc[k];
+        const double qk = quot_near(s[k], den, rden, rden, badc);
+        d[k] = FWD ? qk : in5[k] - qk;
       }
-      t.P = BATCH ? *Pc : P0;
-      exact_cell<W, FWD, MX>(x.p, x.ns, reinterpret_cast<const uint32_t *>(pnb), pslot, prec, qnb,
-                             src, ring, den, limited, t);
-#pragma unroll
-      for (int k = 0; k < 5; k++) d[k] = t.d[k];
-    }
-    if (h == 0 && live) {
-      double2 *rr =
-          reinterpret_cast<double2 *>(ring + ((x.p - pbase) & (kRing - 1)) * kRingRow);
-      rr[0] = make_double2(d[0], d[1]);
-      rr[1] = make_double2(d[2], d[3]);
-      rr[2] = make_double2(d[4], 0.0);
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&lbar[sg % kLevelBars], arrivals);
-    // off the chain: the increment for the other chunks, the other sweep's
-    // sentinel, and in the backward sweep the state update
-    if (live && h == 0) {
-      store_dq(dst, c, d);
-      store_sentinel(rearm, c);  // armed for the other sweep
-      if (FWD && lim > 0.0) {
-        dt[c] = lim;
-        diag[c] = den;
+      double qc[Q_STRIDE], vv;
+      {
+        const double2 a = own[g], b = own[kCells + g], e = own[2 * kCells + g];
+        qc[0] = a.x; qc[1] = a.y; qc[2] = b.x; qc[3] = b.y; qc[4] = e.x;
+        vv = e.y;
       }
-      if (!FWD) {
-        const Params &P = BATCH ? *Pc : P0;
-        update_cell(qc, d, P);
-        cell_props(qc, P);
-        store_q(q8_new, c, qc);
-        if (MX) store_q4(q4_new, c, qc);
-      }
-    }
-  }
-}
-
-// Forward sweep.  chunk_skip > 0 withholds the first chunk_skip chunks
-// (failure-detection self-test only: the cells that depend on them wait
-// until the bound runs out).
-template <int W, bool MX, bool BATCH>
-__global__ void __launch_bounds__(kSweepThreads, 1)
-k_sweep_fwd_chunk(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
-                  const PosCell *__restrict__ pcs,
-                  const typename SweepTypes<MX>::Rec *__restrict__ prec,
-                  const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
-                  const double *__restrict__ q8,
-                  const typename SweepTypes<MX>::Q *__restrict__ qnb, double *dqf,
-                  double *dqb, const double *__restrict__ res, int32_t C,
-                  double *diag, int32_t first_cell, Params P0, int clamp_check,
-                  double *dt, const unsigned long long *__restrict__ dt_ext,
-                  const int32_t *__restrict__ cptr, const SlotRec *__restrict__ slots,
-                  const double *__restrict__ vol, int *err, long long spin,
-                  int32_t chunk_skip, Cases cs) {
-  if ((int32_t)blockIdx.x < chunk_skip) return;
-  chunk_sweep<W, true, MX, BATCH>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqf, dqf, dqb,
-                                  res, nullptr, C, diag, first_cell, P0, clamp_check, dt, dt_ext,
-                                  cptr, slots, vol, err, spin, cs, nullptr, nullptr);
-}
-
-// Backward sweep with the state update (see the section comment).
-template <int W, bool MX, bool BATCH>
-__global__ void __launch_bounds__(kSweepThreads, 1)
-k_sweep_bwd_chunk(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
-                  const PosCell *__restrict__ pcs,
-                  const typename SweepTypes<MX>::Rec *__restrict__ prec,
-                  const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
-                  const double *__restrict__ q8,
-                  const typename SweepTypes<MX>::Q *__restrict__ qnb,
-                  double *__restrict__ q8_new, float *__restrict__ q4_new,
-                  double *dqf, double *dqb, const double *__restrict__ diag,
-                  Params P0, int *err, long long spin, Cases cs) {
-  chunk_sweep<W, false, MX, BATCH>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqb, dqb, dqf,
-                                   nullptr, dqf, 0, const_cast<double *>(diag), 0, P0, 0, nullptr,
-                                   nullptr, nullptr, nullptr, nullptr, err, spin, cs, q8_new,
-                                   q4_new);
-}
-
-// ---------------------------------------------------------------------------
-// Persistent chunked sweeps for wide levels.  The same tables with many
-// small chunks -- several blocks of 64 threads per SM, kWideRing positions
-// in each block's ring -- so that a level of many cells is spread over many
-// blocks and an SM hides one block's waits behind another's work.  A cell is
-// swept by a group of W lanes: lane j computes the flux of record j and owns
-// the components k = j, j + W, ... < 5 of the increment (the ordered sum over
-// the records and the division); every lane applies the limiter.  The
-// operations and their order per component are those of the one-thread
-// form, so the results are the same bits.  A block walks its chunk level by
-// level with __syncthreads between levels; a group's work items (level,
-// pass) are pipelined: indices loaded two items ahead, the read-only data
-// staged into shared memory by cp.async one item ahead.
-// ---------------------------------------------------------------------------
-constexpr int kWideBlock = 64;  // threads per block
-constexpr int kWideMinB = 6;    // resident blocks per SM (register cap)
-constexpr int kWideRing = 128;  // positions of a block's ring
-static_assert((kWideRing & (kWideRing - 1)) == 0, "ring size must be a power of two");
-
-// What a lane knows about its group's position on a future level: the
-// position, its ring slot, the cell, the record count, this lane's
-// neighbours (flags kMark / kInRing) and their ring slots; cell < 0 = none.
-template <int R>
-struct WideRegs {
-  int32_t p, slot, cell, ns;
-  uint32_t nb[R];
-  int32_t nslot[R];
-};
-
-// Everything a group reads for one cell that no sweep writes, staged into
-// shared memory by cp.async one item ahead: neighbour states and records
-// (by the lane of the record), the cell's state and Diag (lane 0), and res
-// (forward) or the cell's forward increment (backward), component k by the
-// lane that owns it.  The mixed form (MX) stages the single-precision
-// neighbour records.
-// Padding of a stage so that consecutive groups' stages start 16 bytes
-// apart modulo 128: the groups of a warp then read their records from
-// different shared-memory banks (without it every group's record k sits in
-// the same bank and a warp's stage reads are 4- to 8-way conflicts).
-constexpr int wide_pad_bytes(int raw) {
-  const int a16 = (raw + 15) / 16 * 16;
-  return a16 - raw + ((16 - a16 % 128) % 128 + 128) % 128;
-}
-template <int W, bool MX>
-struct __align__(16) WideStage {
-  typename SweepTypes<MX>::Q qn[W][Q_STRIDE];
-  typename SweepTypes<MX>::Rec rec[W];
-  double qc[Q_STRIDE];
-  double in5[5];
-  double diag;
-  char pad[wide_pad_bytes(int(sizeof(typename SweepTypes<MX>::Q)) * W * Q_STRIDE +
-                           int(sizeof(typename SweepTypes<MX>::Rec)) * W + 8 * (Q_STRIDE + 6))];
-};
-static_assert(sizeof(WideStage<4, false>) % 128 == 16 && sizeof(WideStage<4, true>) % 128 == 16 &&
-                  sizeof(WideStage<8, false>) % 128 == 16 && sizeof(WideStage<8, true>) % 128 == 16,
-              "stage stride");
-
-template <int W, int L>
-__device__ __forceinline__ void wide_fetch(const int32_t *s_segs, const int32_t *__restrict__ segs,
-                                           int32_t sg0, int32_t sg, int32_t sg1, int32_t pbase,
-                                           int32_t pos_in_level, int32_t lane,
-                                           const PosCell *__restrict__ pcs,
-                                           const int32_t *__restrict__ pnb,
-                                           const int32_t *__restrict__ pslot,
-                                           WideRegs<W / L> &o) {
-  o.cell = -1;
-  o.ns = 0;
+      badc |= dq_over_limit(qc, vv, d, CP) & limits;
+      if (h == 0 && live) bad |= badc;
+      if (__any_sync(0xffffffffu, bad < 0) && h == 0 && live) {
+        ExactArgs t;  // copies, so that the arrays above stay in registers
 #pragma unroll
-  for (int r = 0; r < W / L; r++) {
-    o.nb[r] = 0;
-    o.nslot[r] = 0;
-  }
-  if (sg >= sg1) return;
-  const int32_t i = sg - sg0;
-  const int32_t a = i < kSegCache ? s_segs[i] : segs[sg];
-  const int32_t b = i + 1 <= kSegCache ? s_segs[i + 1] : segs[sg + 1];
-  const int32_t p = a + pos_in_level;
-  if (p >= b) return;
-  const PosCell x = pcs[p];
-  o.p = p;
-  o.slot = (p - pbase) & (kWideRing - 1);
-  o.cell = x.cell;
-  o.ns = x.ns;
-#pragma unroll
-  for (int r = 0; r < W / L; r++) {  // padding reads 0
-    o.nb[r] = (uint32_t)pnb[(int64_t)p * W + lane + L * r];
-    o.nslot[r] = pslot[(int64_t)p * W + lane + L * r];
-  }
-}
-
-template <int W, int L, bool FWD, bool MX>
-__device__ __forceinline__ void wide_stage_copy(const WideRegs<W / L> &o, int32_t lane,
-                                           WideStage<W, MX> &st, const double *q8,
-                                           const typename SweepTypes<MX>::Q *qnb,
-                                           const typename SweepTypes<MX>::Rec *prec,
-                                           const double *res, const double *diag,
-                                           const double *dqf, int32_t C) {
-  if (o.cell < 0) return;
-  // 16-byte pieces of the neighbour record (64 B FP64, 32 B FP32) and of the
-  // sweep record (32 B, 16 B)
-  constexpr int kQ = sizeof(st.qn[0]) / 16, kR = sizeof(st.rec[0]) / 16;
-#pragma unroll
-  for (int r = 0; r < W / L; r++) {
-    const int j = lane + L * r;
-    if (j < o.ns) {
-      const char *qs =
-          reinterpret_cast<const char *>(qnb + (int64_t)(o.nb[r] & kIdMask) * Q_STRIDE);
-      char *qd = reinterpret_cast<char *>(&st.qn[j][0]);
-#pragma unroll
-      for (int i = 0; i < kQ; i++) cp_async16(qd + 16 * i, qs + 16 * i);
-      const char *rs = reinterpret_cast<const char *>(prec + (int64_t)o.p * W + j);
-      char *rd = reinterpret_cast<char *>(&st.rec[j]);
-#pragma unroll
-      for (int i = 0; i < kR; i++) cp_async16(rd + 16 * i, rs + 16 * i);
-    }
-  }
-  if (lane == 0) {
-    const double *qs = q8 + (int64_t)o.cell * Q_STRIDE;
-#pragma unroll
-    for (int i = 0; i < 4; i++) cp_async16(&st.qc[2 * i], qs + 2 * i);
-    cp_async8(&st.diag, diag + o.cell);
-  }
-  for (int k = lane; k < 5; k += L)
-    cp_async8(&st.in5[k], FWD ? res + (int64_t)k * C + o.cell : dqf + (int64_t)o.cell * Q_STRIDE + k);
-}
-
-// One cell of one sweep level on a lane group, from its stage (the group's
-// lanes only wait for one another: a cell is stored as soon as its own
-// inputs are in).  sh: the group's scratch (W * 5 + 5 doubles); ring: the
-// block's increments of its last kWideRing positions.  FWD: DQ* = (res - sum_j
-// 0.5 area_j F_j) / Diag, limited except for the first cell (SolveLUSGS3D
-// forward, forward_lusgs.cpp:799-870); backward: DQ = DQ* - (sum_j area_j
-// F_j) / (2 Diag), limited (:871-940).
-template <int W, int L, bool FWD, bool MX>
-__device__ __forceinline__ void wide_cell(
-    const WideRegs<W / L> &o, int32_t lane, const WideStage<W, MX> &st, double *sh, double *ring,
-    const double (*pre)[5],
-    const double *src, double *dst, double *rearm, int32_t first_cell, const Params &P0,
-    const double *s_lim, int clamp_check, double *__restrict__ dt, double *__restrict__ diag,
-    const unsigned long long *__restrict__ dt_ext, const int32_t *__restrict__ cptr,
-    const SlotRec *__restrict__ slots, const double *__restrict__ vol, int *err,
-    long long spin, const Cases &cs) {
-  if (o.cell < 0) return;  // the whole group
-  const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
-  const int32_t c = o.cell;
-  const int32_t cse = case_of(cs, c);
-  const Params P = params_of(P0, cs, c);
-  // what the cell's own staged data give, formed while its neighbours'
-  // increments are still awaited: the reciprocal of the diagonal term the
-  // increment is divided by, and the velocity square of the limiter
-  const double den = FWD ? st.diag : 2.0 * st.diag;
-  const double rden = 1.0 / den;
-  const double vv = st.qc[1] * st.qc[1] + st.qc[2] * st.qc[2] + st.qc[3] * st.qc[3];
-  // record j = lane + L r < ns: w_j * FluxLUSGS3D(q[nb_j], DQ[nb_j], n_j)
-#pragma unroll
-  for (int r = 0; r < W / L; r++) {
-    const int j = lane + L * r;
-    if (j < o.ns) {
-      const uint32_t b = o.nb[r];
-      // FP64: the part of the product the neighbour's state and the face
-      // give, before the increment is waited for
-      LusgsPre<double> a{};
-      if constexpr (!MX) {
-        double qn[Q_STRIDE];
-#pragma unroll
-        for (int k = 0; k < Q_STRIDE; k++) qn[k] = st.qn[j][k];
-        a = flux_lusgs_pre(qn, st.rec[j].nx, st.rec[j].ny, st.rec[j].nz, flux_params<double>(P));
-      }
-      double dn[5];
-      if (b & kInRing) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) dn[k] = ring[o.nslot[r] * 5 + k];
-      } else if ((b & kMark) && !rec5_ready(pre[r])) {
-        wait_rec(src + (int64_t)(b & kIdMask) * Q_STRIDE, dn, err, spin);
-      } else {  // read at the start of the item (see wide_chunk)
-#pragma unroll
-        for (int k = 0; k < 5; k++) dn[k] = pre[r][k];
-      }
-      if constexpr (MX) {
-        // off-diagonal product in FP32, accumulated in FP64 below
-        float qf[Q_STRIDE], df[5], ff[5];
-#pragma unroll
-        for (int k = 0; k < Q_STRIDE; k++) qf[k] = st.qn[j][k];
-#pragma unroll
-        for (int k = 0; k < 5; k++) df[k] = (float)dn[k];
-        const SweepRecF rr = st.rec[j];
-        flux_lusgs_diff(qf, df, rr.nx, rr.ny, rr.nz, flux_params<float>(P), ff);
-#pragma unroll
-        for (int k = 0; k < 5; k++) sh[j * 5 + k] = (double)(rr.w * ff[k]);
-      } else {
-        double f[5];
-        const SweepRec rr = st.rec[j];
-        flux_lusgs_fin(a, dn, rr.nx, rr.ny, rr.nz, flux_params<double>(P), f);
-#pragma unroll
-        for (int k = 0; k < 5; k++) sh[j * 5 + k] = rr.w * f[k];
-      }
-    }
-  }
-  // LimitTimeStep's clamp (fused forward sweep, and only when some case's
-  // dt ratio exceeds its limit): every component lane reads dt[c] before
-  // lane 0 may write it below
-  double dg = st.diag, lim = -1.0;
-  bool clamped = false;
-  if (FWD && clamp_check && lane < 5) {
-    lim = (cse < kCaseCache) ? s_lim[cse] : clamp_limit(P, dt_ext + 2 * cse);
-    if (lim > 0.0 && dt[c] > lim) {
-      double qc[Q_STRIDE];
-#pragma unroll
-      for (int i = 0; i < Q_STRIDE; i++) qc[i] = st.qc[i];
-      dg = clamped_diag(c, qc, P, lim, cptr, slots, vol);
-      clamped = true;
-    }
-  }
-  __syncwarp(gmask);
-  // components k = lane, lane + L, ... < 5 (at most two per lane, as two
-  // independent chains); records summed in order
-  {
-    constexpr int kC = (5 + L - 1) / L;
-    double acc[kC];
-#pragma unroll
-    for (int i = 0; i < kC; i++) {
-      const int k = lane + L * i;
-      acc[i] = (FWD && k < 5) ? st.in5[k] : 0.0;
-    }
-    for (int32_t j = 0; j < o.ns; j++) {
-#pragma unroll
-      for (int i = 0; i < kC; i++) {
-        const int k = lane + L * i;
-        if (k < 5) {
-          if (FWD)
-            acc[i] -= sh[j * 5 + k];
-          else
-            acc[i] += sh[j * 5 + k];
+        for (int k = 0; k < 5; k++) {
+          t.in5[k] = in5[k];
+          t.qc[k] = qc[k];
         }
+        t.P = BATCH ? *Pc : P0;
+        exact_cell<W, FWD, MX>(x.p, ns, pnb, prec, qnb, src, ring, den, limits != 0, t);
+#pragma unroll
+        for (int k = 0; k < 5; k++) d[k] = t.d[k];
       }
-    }
-#pragma unroll
-    for (int i = 0; i < kC; i++) {
-      const int k = lane + L * i;
-      if (k < 5)
-        sh[W * 5 + k] = FWD ? (clamped ? acc[i] / dg : div_by_recip(acc[i], den, rden))
-                            : st.in5[k] - div_by_recip(acc[i], den, rden);
-    }
-  }
-  __syncwarp(gmask);
-  // the limiter on every lane (same values), the stores spread over the lanes
-  double d[5], qc[Q_STRIDE];
-#pragma unroll
-  for (int k = 0; k < 5; k++) d[k] = sh[W * 5 + k];
-#pragma unroll
-  for (int i = 0; i < Q_STRIDE; i++) qc[i] = st.qc[i];
-  if (!FWD || c != (cs.P ? cs.first[cse] : first_cell)) dq_limit_vv(qc, vv, d, P);
-  if (lane == 0) {
-    if (FWD && clamped) {
-      dt[c] = lim;
-      diag[c] = dg;
-    }
-    store_dq(dst, c, d);
-  }
-  if (lane == (L > 1 ? 1 : 0)) store_sentinel(rearm, c);  // armed for the other sweep
-#pragma unroll
-  for (int k = 0; k < 5; k++)
-    if (k % L == lane) ring[o.slot * 5 + k] = d[k];
-  __syncwarp(gmask);  // sh is free for the group's next cell
-}
-
-// One persistent sweep: block b walks chunk b level by level.  A level of
-// more cells than the block has groups takes several passes; the group's
-// work items (level, pass) form one sequence, pipelined as a whole: indices
-// loaded two items ahead, read-only data staged into shared memory one item
-// ahead (cp.async), so that an item's critical path holds the increments it
-// depends on and one cell's arithmetic.  Blocks synchronise only between
-// levels.
-template <int W, int L, bool FWD, bool MX>
-__device__ __forceinline__ void wide_chunk(
-    const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
-    const PosCell *__restrict__ pcs, const typename SweepTypes<MX>::Rec *__restrict__ prec,
-    const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
-    const double *__restrict__ q8, const typename SweepTypes<MX>::Q *__restrict__ qnb,
-    const double *src, double *dst, double *rearm,
-    const double *__restrict__ res, const double *__restrict__ dqf_own, int32_t C,
-    double *__restrict__ diag, int32_t first_cell, const Params &P0, int clamp_check,
-    double *__restrict__ dt, const unsigned long long *__restrict__ dt_ext,
-    const int32_t *__restrict__ cptr, const SlotRec *__restrict__ slots,
-    const double *__restrict__ vol, int *err, long long spin, const Cases &cs) {
-  constexpr int kGroups = kWideBlock / L;
-  __shared__ WideStage<W, MX> stg[2][kGroups];
-  __shared__ double shm[kGroups][W * 5 + 5];
-  __shared__ double ring[kWideRing * 5];
-  __shared__ int32_t s_segs[kSegCache + 1];
-  __shared__ double s_lim[FWD ? kCaseCache : 1];
-  const int32_t sg0 = seg_begin[blockIdx.x], sg1 = seg_begin[blockIdx.x + 1];
-  const int32_t lane = threadIdx.x & (L - 1);
-  const int32_t grp = threadIdx.x / L;
-  for (int32_t i = threadIdx.x; i <= sg1 - sg0 && i <= kSegCache; i += blockDim.x)
-    s_segs[i] = segs[sg0 + i];
-  __shared__ int s_clamp_any;
-  if (threadIdx.x == 0) s_clamp_any = 0;
-  __syncthreads();
-  if (FWD && clamp_check)
-    for (int32_t k = threadIdx.x; k < cs.ncase && k < kCaseCache; k += blockDim.x) {
-      s_lim[k] = clamp_limit(cs.P ? cs.P[k] : P0, dt_ext + 2 * k);
-      if (s_lim[k] > 0.0) s_clamp_any = 1;
-    }
-  if (FWD && clamp_check && cs.ncase > kCaseCache && threadIdx.x == 0) s_clamp_any = 1;
-  __syncthreads();
-  // the per-cell clamp test only when some case needs it
-  clamp_check = (FWD && clamp_check && s_clamp_any) ? 1 : 0;
-  const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
-  double *sh = shm[grp];
-  const int32_t pbase = sg1 > sg0 ? s_segs[0] : 0;
-  // work items (level sg, pass): the same sequence in every thread of the block
-  auto seg_at = [&](int32_t sg) {
-    const int32_t i = sg - sg0;
-    return i <= kSegCache ? s_segs[i] : segs[sg];
-  };
-  auto advance = [&](int32_t &sg, int32_t &pass) {
-    if (sg >= sg1) return;
-    const int32_t np = (seg_at(sg + 1) - seg_at(sg) + kGroups - 1) / kGroups;
-    if (++pass >= np) {
-      ++sg;
-      pass = 0;
-    }
-  };
-  auto fetch = [&](int32_t sg, int32_t pass, WideRegs<W / L> &o) {
-    wide_fetch<W, L>(s_segs, segs, sg0, sg, sg1, pbase, grp + pass * kGroups, lane, pcs, pnb,
-                     pslot, o);
-  };
-  int32_t sg = sg0, pass = 0;              // this item
-  int32_t sgn = sg, passn = pass;          // the next
-  advance(sgn, passn);
-  int32_t sgf = sgn, passf = passn;        // the one after
-  advance(sgf, passf);
-  WideRegs<W / L> cur, nxt, far;
-  fetch(sg, pass, cur);
-  fetch(sgn, passn, nxt);
-  wide_stage_copy<W, L, FWD, MX>(cur, lane, stg[0][grp], q8, qnb, prec, res, diag, dqf_own, C);
-  cp_async_commit();
-  int par = 0;
-  while (sg < sg1) {
-    // increments this item reads from L2 (older than the ring, or produced by
-    // another chunk): requested first, so that their round trip overlaps the
-    // staging of the next items; one that still holds the sentinel is waited
-    // for in wide_cell
-    double pre[W / L][5];
-#pragma unroll
-    for (int r = 0; r < W / L; r++) {
-      const int j = lane + L * r;
-      if (cur.cell >= 0 && j < cur.ns && !(cur.nb[r] & kInRing))
-        load_rec5_l2(src + (int64_t)(cur.nb[r] & kIdMask) * Q_STRIDE, pre[r]);
-    }
-    fetch(sgf, passf, far);
-    wide_stage_copy<W, L, FWD, MX>(nxt, lane, stg[par ^ 1][grp], q8, qnb, prec, res, diag, dqf_own,
-                              C);
-    cp_async_commit();
-    cp_async_wait<1>();  // this item's stage
-    __syncwarp(gmask);
-    wide_cell<W, L, FWD, MX>(cur, lane, stg[par][grp], sh, ring, pre, src, dst, rearm, first_cell,
-                              P0, s_lim, clamp_check, dt, diag, dt_ext, cptr, slots, vol, err,
-                              spin, cs);
-    if (sgn != sg) __syncthreads();  // end of a level
-    sg = sgn;
-    pass = passn;
-    sgn = sgf;
-    passn = passf;
-    advance(sgf, passf);
-    cur = nxt;
-    nxt = far;
-    par ^= 1;
+      if (h == 0 && live) {
+        double2 *rr =
+            reinterpret_cast<double2 *>(ring + ((x.p - pbase) & (kRing - 1)) * kRingRow);
+        rr[0] = make_double2(d[0], d[1]);
+        rr[1] = make_double2(d[2], d[3]);
+        rr[2] = make_double2(d[4], 0.0);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&lbar[sg % kLevelBars], x.arrivals);
+      // off the chain: the increment's row, and the other sweep's sentinel
+      // (both in the same stores, by the cell's first two lanes)
+      if (live && (h == 0 || (h == 1 && arm))) {
+        const double sn = __longlong_as_double((long long)kSentinelBits);
+        double *to = (h ? rearm : dst) + (int64_t)c * Q_STRIDE;
+        stg_v4(to, h ? sn : d[0], h ? sn : d[1], h ? sn : d[2], h ? sn : d[3]);
+        *reinterpret_cast<double2 *>(to + 4) = make_double2(h ? sn : d[4], 0.0);
+      }
+    };
+    // most items have no lane with a second record: positions are sorted by
+    // record count within a level
+    if (__any_sync(0xffffffffu, ns > L))
+      turn(std::integral_constant<int, R>());
+    else
+      turn(std::integral_constant<int, 1>());
   }
   cp_async_wait<0>();
 }
@@ -2017,52 +1663,45 @@ __device__ __forceinline__ void wide_chunk(
 // Forward sweep.  chunk_skip > 0 withholds the first chunk_skip chunks
 // (failure-detection self-test only: the cells that depend on them wait
 // until the bound runs out).
-template <int W, int L, bool MX>
-__global__ void __launch_bounds__(kWideBlock, kWideMinB)
-k_sweep_fwd_wide(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
-                  const PosCell *__restrict__ pcs,
+template <int W, bool MX, bool BATCH, int NW>
+__global__ void __launch_bounds__(32 * NW, kSweepWarps / NW)
+k_sweep_fwd_chunk(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
+                  const int32_t *__restrict__ seg_items, const PosCell *__restrict__ pcs,
                   const typename SweepTypes<MX>::Rec *__restrict__ prec,
-                  const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
-                  const double *__restrict__ q8,
-                  const typename SweepTypes<MX>::Q *__restrict__ qnb, double *dqf,
-                  double *__restrict__ dqb, const double *__restrict__ res, int32_t C,
-                  double *__restrict__ diag, int32_t first_cell, Params P0, int clamp_check,
-                  double *__restrict__ dt, const unsigned long long *__restrict__ dt_ext,
+                  const SweepNb *__restrict__ pnb, const double *__restrict__ q8,
+                  const typename SweepTypes<MX>::Q *__restrict__ qnb, double *dqf, double *dqb,
+                  const double *__restrict__ res, int32_t C, double *diag, int32_t first_cell,
+                  Params P0, int clamp_check, double *dt,
+                  const unsigned long long *__restrict__ dt_ext,
                   const int32_t *__restrict__ cptr, const SlotRec *__restrict__ slots,
-                  const double *__restrict__ vol, int *err, long long spin,
-                  int32_t chunk_skip, Cases cs) {
+                  const double *__restrict__ vol, int *err, long long spin, int32_t chunk_skip,
+                  Cases cs) {
   if ((int32_t)blockIdx.x < chunk_skip) return;
-  wide_chunk<W, L, true, MX>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqf, dqf, dqb, res,
-                              nullptr, C, diag, first_cell, P0, clamp_check, dt, dt_ext, cptr,
-                              slots, vol, err, spin, cs);
+  chunk_sweep<W, true, MX, BATCH, NW>(seg_begin, segs, seg_items, pcs, prec, pnb, q8, qnb,
+                                      dqf, dqf, dqb, res, nullptr, C, diag, first_cell, P0,
+                                      clamp_check, dt, dt_ext, cptr, slots, vol, err, spin, cs);
 }
 
-// Backward sweep.  The state update is k_update_cells, launched after it:
-// a separate streaming pass reads each cell's state and increment once in
-// cell order, where an update by each block after its chunk (cells in
-// chunk order, one after another per thread) took 0.79 ms of the 128^3
-// iteration against 0.35 ms.  q8_new and q4_new are unused here (the
-// argument list is the deep kernels').
-template <int W, int L, bool MX>
-__global__ void __launch_bounds__(kWideBlock, kWideMinB)
-k_sweep_bwd_wide(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
-                  const PosCell *__restrict__ pcs,
+// Backward sweep.  The state update is k_update_cells, launched after it: by
+// the warps of the sweep it lengthened every turn (64^3 x 6 cells: 367 us for
+// the sweep with the update in it, 339 with the pass).
+template <int W, bool MX, bool BATCH, int NW>
+__global__ void __launch_bounds__(32 * NW, kSweepWarps / NW)
+k_sweep_bwd_chunk(const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
+                  const int32_t *__restrict__ seg_items, const PosCell *__restrict__ pcs,
                   const typename SweepTypes<MX>::Rec *__restrict__ prec,
-                  const int32_t *__restrict__ pnb, const int32_t *__restrict__ pslot,
-                  const double *__restrict__ q8,
-                  const typename SweepTypes<MX>::Q *__restrict__ qnb,
-                  double *__restrict__ q8_new, float *__restrict__ q4_new,
-                  double *__restrict__ dqf, double *dqb, const double *__restrict__ diag,
-                  Params P0, int *err, long long spin, Cases cs) {
-  wide_chunk<W, L, false, MX>(seg_begin, segs, pcs, prec, pnb, pslot, q8, qnb, dqb, dqb, dqf,
-                               nullptr, dqf, 0, const_cast<double *>(diag), 0, P0, 0, nullptr,
-                               nullptr, nullptr, nullptr, nullptr, err, spin, cs);
+                  const SweepNb *__restrict__ pnb, const double *__restrict__ q8,
+                  const typename SweepTypes<MX>::Q *__restrict__ qnb, double *dqf, double *dqb,
+                  double *diag, Params P0, int *err, long long spin, Cases cs) {
+  chunk_sweep<W, false, MX, BATCH, NW>(seg_begin, segs, seg_items, pcs, prec, pnb, q8, qnb,
+                                       dqb, dqb, dqf, nullptr, dqf, 0, diag, 0, P0, 0, nullptr,
+                                       nullptr, nullptr, nullptr, nullptr, err, spin, cs);
 }
 
 // UpdateFlowField3D_CFL3d (forward_lusgs.cpp:1335-1488) of every cell from
 // its state and backward increment, the new state (with a, H, E; and the
 // single-precision record of the mixed form) into the other state buffer:
-// the update of the wide backward sweeps, one thread per cell.
+// the update of the backward sweeps, one thread per cell.
 template <bool MX>
 __global__ void __launch_bounds__(kBlock)
 k_update_cells(int32_t C, const double *__restrict__ q8, const double *__restrict__ dqb,
@@ -2709,10 +2348,12 @@ __global__ void k_selftest_functions(int mode, int32_t n, Params P, const double
     cell_props(q, P);
     const FluxP<double> fp = flux_params<double>(P);
     const LusgsPre<double> a = flux_lusgs_pre(q, c[10], c[11], c[12], fp);
-    bool ok = false;
-    if (mode == 3)
-      flux_lusgs_fin_near(a, rcp_seed(q[0]), dq, c[10], c[11], c[12], fp, f, ok);
-    if (!ok) flux_lusgs_fin(a, dq, c[10], c[11], c[12], fp, f);
+    int bad = -1;
+    if (mode == 3) {
+      bad = 0;
+      flux_lusgs_fin_near(a, rcp_seed(q[0]), dq, c[10], c[11], c[12], fp, f, bad);
+    }
+    if (bad < 0) flux_lusgs_fin(a, dq, c[10], c[11], c[12], fp, f);
     for (int k = 0; k < 5; k++) out[5 * (int64_t)i + k] = f[k];
   } else {
     double q[Q_STRIDE], dq[5];
@@ -2762,16 +2403,16 @@ __global__ void k_selftest_division_fast(int64_t n, uint64_t seed,
     // from the seed of a divisor within 1/16 of b
     const double b0f = b * (1.0 + ((double)(int64_t)(ra >> 12) * 0x1p-52 - 0.5) * 0.115);
     double near;
-    bool okn;
-    const double yn = rcp_rn_near(b, __hiloint2double(rcp_seed(b0f), 0), near, okn);
-    if (!okn) {
+    int badn = 0, badq = 0, badz = 0;
+    const double yn = rcp_rn_near(b, __hiloint2double(rcp_seed(b0f), 0), near, badn);
+    if (badn < 0) {
       if (fabs(b) > 0x1p-119 && fabs(b) < 0x1p119) b0++;  // inside the window
     } else {
       if (__double_as_longlong(yn) != __double_as_longlong(1.0 / b)) b0++;
-      const double qn = div_recip_near(a, b, near, yn, okq);
-      if (okq && __double_as_longlong(qn) != __double_as_longlong(a / b)) b1++;
-      const double z = div_recip_near(0.0, b, near, yn, okq);
-      if (!okq || __double_as_longlong(z) != __double_as_longlong(0.0 / b)) b1++;
+      const double qn = quot_near(a, b, near, yn, badq);
+      if (badq >= 0 && __double_as_longlong(qn) != __double_as_longlong(a / b)) b1++;
+      const double z = copysign(0.0, a), qz = quot_near(z, b, near, yn, badz);
+      if (badz < 0 || __double_as_longlong(qz) != __double_as_longlong(z / b)) b1++;
     }
   }
   if (b0) atomicAdd(bad, b0);
@@ -2921,43 +2562,53 @@ __global__ void k_halo_nodes_mx(int32_t nu, const int32_t *__restrict__ unodes,
 // context
 // ---------------------------------------------------------------------------
 
-// The persistent sweep kernel for (W, precision, one grid or a batch).
-// kind MFG_SWEEP_DEEP: one block per SM; MFG_SWEEP_WIDE: the many-block
-// kernels for wide levels.
-static const void *sweep_kernel(bool fwd, int w, bool mx, bool batch, int kind = MFG_SWEEP_DEEP) {
-#define MFG_SK(W_, MX_)                                                                     \
-  if (w == W_ && mx == MX_ && kind == MFG_SWEEP_DEEP)                                        \
-    return fwd ? (batch ? (const void *)k_sweep_fwd_chunk<W_, MX_, true>                      \
-                        : (const void *)k_sweep_fwd_chunk<W_, MX_, false>)                    \
-               : (batch ? (const void *)k_sweep_bwd_chunk<W_, MX_, true>                      \
-                        : (const void *)k_sweep_bwd_chunk<W_, MX_, false>);                   \
-  if (w == W_ && mx == MX_ && kind == MFG_SWEEP_WIDE)                                        \
-    return fwd ? (const void *)k_sweep_fwd_wide<W_, W_, MX_>                                  \
-               : (const void *)k_sweep_bwd_wide<W_, W_, MX_>;
-  MFG_SK(4, false)
-  MFG_SK(4, true)
-  MFG_SK(8, false)
-  MFG_SK(8, true)
-#undef MFG_SK
+// The persistent sweep kernel for (W, precision, one grid or a batch), in one
+// block of kSweepWarps warps per SM (MFG_SWEEP_DEEP) or two of half as many
+// (MFG_SWEEP_WIDE).
+template <int W, bool MX, bool BATCH, int NW>
+static const void *sweep_kernel_of(bool fwd) {
+  return fwd ? (const void *)k_sweep_fwd_chunk<W, MX, BATCH, NW>
+             : (const void *)k_sweep_bwd_chunk<W, MX, BATCH, NW>;
+}
+template <int W, bool MX>
+static const void *sweep_kernel_of(bool fwd, bool batch, int kind) {
+  if (kind == MFG_SWEEP_WIDE)
+    return batch ? sweep_kernel_of<W, MX, true, kSweepWarps / 2>(fwd)
+                 : sweep_kernel_of<W, MX, false, kSweepWarps / 2>(fwd);
+  return batch ? sweep_kernel_of<W, MX, true, kSweepWarps>(fwd)
+               : sweep_kernel_of<W, MX, false, kSweepWarps>(fwd);
+}
+static const void *sweep_kernel(bool fwd, int w, bool mx, bool batch, int kind) {
+  if (w == 4)
+    return mx ? sweep_kernel_of<4, true>(fwd, batch, kind)
+              : sweep_kernel_of<4, false>(fwd, batch, kind);
+  if (w == 8)
+    return mx ? sweep_kernel_of<8, true>(fwd, batch, kind)
+              : sweep_kernel_of<8, false>(fwd, batch, kind);
   return nullptr;
 }
 static int sweep_threads(int kind) {
-  return kind == MFG_SWEEP_WIDE ? kWideBlock : kSweepThreads;
+  return 32 * (kind == MFG_SWEEP_WIDE ? kSweepWarps / 2 : kSweepWarps);
 }
 static size_t sweep_smem(int w, int kind) {
-  if (kind == MFG_SWEEP_WIDE) return 0;
-  return w == 8 ? sweep_smem_bytes<8>() : sweep_smem_bytes<4>();
+  if (kind == MFG_SWEEP_WIDE)
+    return w == 8 ? sweep_smem_bytes<8, kSweepWarps / 2>() : sweep_smem_bytes<4, kSweepWarps / 2>();
+  return w == 8 ? sweep_smem_bytes<8, kSweepWarps>() : sweep_smem_bytes<4, kSweepWarps>();
 }
-// Cells of a level that a kernel kind's block sweeps side by side (as the
-// chunk model counts them), and the ring positions of a kind.
-static int32_t sweep_groups(int w, int kind = MFG_SWEEP_DEEP) {
-  if (kind == MFG_SWEEP_WIDE) return kWideBlock / std::max(w, 1);
-  return w == 8 ? 32 : 64;
+// Cells of a level that a kernel kind's block sweeps side by side, as the
+// chunk model counts them.
+static int32_t sweep_groups(int w, int kind) {
+  return (w == 8 ? 32 : 64) / (kind == MFG_SWEEP_WIDE ? 2 : 1);
 }
-static int32_t sweep_ring(int kind) { return kind == MFG_SWEEP_WIDE ? kWideRing : kRing; }
+// Cells of a warp's item in the deep sweeps.
+static int32_t sweep_item_cells(int w) {
+  return w == 8 ? SweepGeom<8>::kCells : SweepGeom<4>::kCells;
+}
 
 struct ChunkSweep {
-  int32_t *seg_begin = nullptr, *segs = nullptr, *nbs = nullptr, *nslots = nullptr;
+  int32_t *seg_begin = nullptr, *segs = nullptr;
+  SweepNb *nbs = nullptr;
+  int32_t *seg_items = nullptr;  // warp items of the deep sweeps before each segment
   PosCell *cells = nullptr;
   SweepRec *recs = nullptr;
   SweepRecF *recs_f = nullptr;  // mixed form
@@ -3358,15 +3009,32 @@ __global__ void k_dev_level_records(int32_t C, const int32_t *__restrict__ cells
   }
 }
 
-// chunk of each level-sorted position (sort key) and its index (value)
-__global__ void k_dev_chunk_keys(int32_t C, const int32_t *__restrict__ cells,
-                                 const int32_t *__restrict__ assign, int32_t *__restrict__ keys,
-                                 int32_t *__restrict__ idx, int32_t *__restrict__ chunk_cnt) {
+// sort keys that put a level's cells of many records first: the record count
+// of each level-sorted position (at most 8 where the tables are read), then,
+// in that order, its level
+__global__ void k_dev_count_keys(int32_t C, const int32_t *__restrict__ sptr,
+                                 int32_t *__restrict__ keys, int32_t *__restrict__ idx) {
   const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= C) return;
-  const int32_t p = assign[cells[i]];
-  keys[i] = p;
+  keys[i] = 8 - min(sptr[i + 1] - sptr[i], 8);
   idx[i] = i;
+}
+__global__ void k_dev_level_keys(int32_t C, const int32_t *__restrict__ cells,
+                                 const int32_t *__restrict__ ord, const int32_t *__restrict__ lvl,
+                                 int32_t *__restrict__ keys) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < C) keys[i] = lvl[cells[ord[i]]];
+}
+
+// chunk of each position in that order (sort key)
+__global__ void k_dev_chunk_keys(int32_t C, const int32_t *__restrict__ cells,
+                                 const int32_t *__restrict__ ord,
+                                 const int32_t *__restrict__ assign, int32_t *__restrict__ keys,
+                                 int32_t *__restrict__ chunk_cnt) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= C) return;
+  const int32_t p = assign[cells[ord[i]]];
+  keys[i] = p;
   atomicAdd(&chunk_cnt[p], 1);
 }
 
@@ -3399,6 +3067,13 @@ __global__ void k_dev_segs(int32_t C, const int32_t *__restrict__ head,
     segs[hscan[k]] = k;
 }
 
+// warp items of each segment (one more entry, 0, for the scan)
+__global__ void k_dev_seg_items(int32_t nseg, int32_t per, const int32_t *__restrict__ segs,
+                                int32_t *__restrict__ cnt) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i <= nseg) cnt[i] = i < nseg ? (segs[i + 1] - segs[i] + per - 1) / per : 0;
+}
+
 __global__ void k_dev_seg_begin(int32_t P, const int32_t *__restrict__ chunk_ptr,
                                 const int32_t *__restrict__ hscan,
                                 int32_t *__restrict__ seg_begin) {
@@ -3415,10 +3090,10 @@ __global__ void k_dev_pack(int32_t C, int32_t W, int with_recs, const int32_t *_
                            const int32_t *__restrict__ posof, const int32_t *__restrict__ assign,
                            const int32_t *__restrict__ sptr, const int32_t *__restrict__ nbs,
                            const SweepRec *__restrict__ recs, PosCell *__restrict__ packed,
-                           int32_t *__restrict__ cnbs, SweepRec *__restrict__ crecs,
-                           SweepRecF *__restrict__ crecs_f, int32_t *__restrict__ cslot,
+                           SweepNb *__restrict__ cnbs, SweepRec *__restrict__ crecs,
+                           SweepRecF *__restrict__ crecs_f,
                            int32_t *__restrict__ chunk0_exported, int32_t *__restrict__ stats,
-                           int32_t ring) {
+                           int32_t ring, uint8_t *__restrict__ from_l2) {
   const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= C) return;
   const int32_t gi = order[k];
@@ -3434,23 +3109,32 @@ __global__ void k_dev_pack(int32_t C, int32_t W, int with_recs, const int32_t *_
     const bool cross = nb < C && assign[nb] != p;
     if (cross && assign[nb] == 0) *chunk0_exported = 1;
     uint32_t e = (uint32_t)nb;
+    int32_t slot = 0;
     if (cross) {
       e |= kMark;
       atomicAdd(&stats[2], 1);
     } else if (nb < C && posof[nb] >= seg_end - ring) {
       e |= kInRing;
-      cslot[o] = (posof[nb] - chunk_ptr[p]) & (ring - 1);
+      slot = (posof[nb] - chunk_ptr[p]) & (ring - 1);
       atomicAdd(&stats[0], 1);
     } else if (nb < C) {
       atomicAdd(&stats[1], 1);
     }
-    cnbs[o] = (int32_t)e;
+    if (nb < C && !(e & kInRing)) from_l2[nb] = 1;
+    cnbs[o] = SweepNb{e, slot};
     const SweepRec r = recs[s0 + j];
     if (MX)
       crecs_f[o] = SweepRecF{(float)r.nx, (float)r.ny, (float)r.nz, (float)r.w};
     else
       crecs[o] = r;
   }
+}
+
+// a cell whose increment the other sweep reads from L2 (kArm)
+__global__ void k_dev_arm(int32_t C, const uint8_t *__restrict__ from_l2,
+                          PosCell *__restrict__ packed) {
+  const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < C && from_l2[packed[k].cell]) packed[k].ns |= kArm;
 }
 
 // build_node_lists' passes (CompNodeVar3D_dist, cal_gradient.cpp:2041-2125,
@@ -3599,15 +3283,9 @@ static void setup_sweep_grid(mfg_ctx *ctx, int32_t maxns, int force_kind = -1) {
     return ctx->sweep_w ? ctx->persist_occ[kind][wi] * ctx->n_sm : 0;
   };
   int kind = force_kind >= 0 ? force_kind : g_sweep_kind.load();
-  if (kind < 0) {
-    const int32_t pdeep = std::max(1, std::min(grid_of(MFG_SWEEP_DEEP), (C + kMinChunk - 1) / kMinChunk));
-    kind = (int64_t)ctx->max_level_cells > 2LL * sweep_groups(ctx->sweep_w) * pdeep
-               ? MFG_SWEEP_WIDE
-               : MFG_SWEEP_DEEP;
-  }
+  if (kind < 0) kind = MFG_SWEEP_DEEP;
   if (grid_of(kind) <= 0) kind = kind == MFG_SWEEP_WIDE ? MFG_SWEEP_DEEP : MFG_SWEEP_WIDE;
   ctx->sweep_kind = kind;
-  ctx->ring = sweep_ring(kind);
   ctx->persist_grid = grid_of(kind);
   ctx->nchunks = std::max(1, std::min(ctx->persist_grid, (C + kMinChunk - 1) / kMinChunk));
   ctx->sweep_mode = ctx->persist_grid > 0 ? 1 : 0;
@@ -3930,6 +3608,9 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
     setup_sweep_grid(ctx, maxns);
   }
   const int W = std::max(ctx->sweep_w, 1);
+  // per sweep: its positions, and the cells whose increments it reads from L2
+  std::vector<PosCell> packed_of[2];
+  std::vector<char> from_l2[2] = {std::vector<char>(C, 0), std::vector<char>(C, 0)};
   auto make = [&](const std::vector<int32_t> &lv, const std::vector<int32_t> &cnt, bool fwd,
                   std::vector<int32_t> &lptr, int32_t **d_cells, int32_t **d_sptr,
                   SweepRec **d_recs, int32_t **d_nb) -> int {
@@ -3982,20 +3663,25 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
     for (int32_t p = 0; p < P; p++) chunk_ptr[p + 1] = chunk_ptr[p] + chunk_cnt[p];
     std::vector<int32_t> slot_of(C), cfill(chunk_ptr.begin(), chunk_ptr.end() - 1);
     std::vector<int32_t> ccells(C);
-    for (int32_t i = 0; i < C; i++) {
-      const int32_t c = cells[i];
-      slot_of[i] = cfill[assign[c]]++;
-      ccells[slot_of[i]] = c;
-    }
+    // a level's cells of many records first, so that a warp's cells have as many
+    for (int32_t l = 0; l + 1 < (int32_t)lptr.size(); l++)
+      for (int32_t k = 8; k >= 0; k--)
+        for (int32_t i = lptr[l]; i < lptr[l + 1]; i++) {
+          const int32_t c = cells[i];
+          if (std::min(cnt[c], 8) != k) continue;
+          slot_of[i] = cfill[assign[c]]++;
+          ccells[slot_of[i]] = c;
+        }
     std::vector<int32_t> gpos(C);
     for (int32_t i = 0; i < C; i++) gpos[cells[i]] = i;
     std::vector<int32_t> segs, seg_begin;
     // position-major: the records of position k at [k * W, k * W + ns)
-    std::vector<int32_t> cnbs((size_t)C * W, 0);
+    std::vector<SweepNb> cnbs((size_t)C * W, SweepNb{0, 0});
     std::vector<SweepRec> crecs((size_t)C * W, SweepRec{0.0, 0.0, 0.0, 0.0});
-    std::vector<int32_t> cslot((size_t)C * W, 0), posof(C);
+    std::vector<int32_t> posof(C);
     for (int32_t k = 0; k < C; k++) posof[ccells[k]] = k;
-    std::vector<PosCell> packed(C);
+    std::vector<PosCell> &packed = packed_of[fwd ? 0 : 1];
+    packed.resize(C);
     bool chunk0_exported = false;
     for (int32_t p = 0; p < P; p++) {
       seg_begin.push_back((int32_t)segs.size());
@@ -4017,6 +3703,7 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
           if (cross && assign[nb] == 0) chunk0_exported = true;
           uint32_t e = (uint32_t)nb;
           int32_t *stat = ctx->sweep_stats[fwd ? 0 : 1];
+          if (nb < C && (cross || posof[nb] < seg_end - ctx->ring)) from_l2[fwd ? 0 : 1][nb] = 1;
           if (cross) {
             e |= kMark;
             stat[2]++;
@@ -4024,12 +3711,12 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
             // still in the ring when this level reads it: overwritten only by
             // position posof[nb] + ring, which lies in a later level
             e |= kInRing;
-            cslot[o] = (posof[nb] - chunk_ptr[p]) & (ctx->ring - 1);
+            cnbs[o].slot = (posof[nb] - chunk_ptr[p]) & (ctx->ring - 1);
             stat[0]++;
           } else if (nb < C) {
             stat[1]++;  // in the chunk, older than the ring: read from global memory
           }
-          cnbs[o] = (int32_t)e;
+          cnbs[o].nb = e;
           crecs[o] = recs[s0];
         }
       }
@@ -4046,7 +3733,11 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
     cs.nseg = (int32_t)segs.size() - 1;
     if ((rc = dupload(ctx, &cs.seg_begin, seg_begin))) return rc;
     if ((rc = dupload(ctx, &cs.segs, segs))) return rc;
-    if ((rc = dupload(ctx, &cs.cells, packed))) return rc;
+    std::vector<int32_t> items(segs.size(), 0);
+    const int32_t per = sweep_item_cells(W);
+    for (size_t i = 0; i + 1 < segs.size(); i++)
+      items[i + 1] = items[i] + (segs[i + 1] - segs[i] + per - 1) / per;
+    if ((rc = dupload(ctx, &cs.seg_items, items))) return rc;
     if (ctx->precision == MFG_PREC_MIXED) {
       std::vector<SweepRecF> rf(crecs.size());
       for (size_t i = 0; i < crecs.size(); i++)
@@ -4057,15 +3748,21 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
       if ((rc = dupload(ctx, &cs.recs, crecs))) return rc;
     }
     if ((rc = dupload(ctx, &cs.nbs, cnbs))) return rc;
-    if ((rc = dupload(ctx, &cs.nslots, cslot))) return rc;
     return MFG_OK;
   };
   (void)n;
   int rc = make(lvl, fw_cnt, true, ctx->fw_lptr, &ctx->fw_cells, &ctx->fw_sptr, &ctx->fw_recs,
                 &ctx->fw_nb);
   if (rc) return rc;
-  return make(blvl, bw_cnt, false, ctx->bw_lptr, &ctx->bw_cells, &ctx->bw_sptr, &ctx->bw_recs,
-              &ctx->bw_nb);
+  if ((rc = make(blvl, bw_cnt, false, ctx->bw_lptr, &ctx->bw_cells, &ctx->bw_sptr, &ctx->bw_recs,
+                 &ctx->bw_nb)))
+    return rc;
+  for (int k = 0; k < 2; k++) {  // each sweep arms the rows that the other reads from L2
+    for (PosCell &x : packed_of[k])
+      if (from_l2[k ^ 1][x.cell]) x.ns |= kArm;
+    if ((rc = dupload(ctx, k ? &ctx->bwc.cells : &ctx->fwc.cells, packed_of[k]))) return rc;
+  }
+  return MFG_OK;
 }
 
 // Node contribution lists that replay CompNodeVar3D_dist's loops
@@ -4680,6 +4377,7 @@ int d2h(std::vector<T> &h, const T *d, int64_t count, cudaStream_t st) {
 struct DevSweep {
   bool fwd = true;
   int32_t *cnt = nullptr, *deg = nullptr, *lvl = nullptr;  // device scratch
+  uint8_t *from_l2 = nullptr;                              // cells read from L2, by dev_pack
   std::vector<int32_t> lptr;                              // level starts
   int32_t L = 0;
   std::vector<int32_t> h_cells, h_sptr, h_nbs, h_assign;  // for the chunk assignment
@@ -4752,8 +4450,8 @@ int dev_pack(mfg_ctx *ctx, DevScratch &sc, DevSweep &d) {
   int rc;
   int32_t *assign = nullptr, *keys = nullptr, *idx = nullptr, *pchunk = nullptr, *order = nullptr;
   int32_t *chunk_cnt = nullptr, *chunk_ptr = nullptr, *ccells = nullptr, *posof = nullptr;
-  int32_t *head = nullptr, *hscan = nullptr, *exported = nullptr;
-  if ((rc = sc.get(&assign, C)) || (rc = sc.get(&keys, C)) || (rc = sc.get(&idx, C)) ||
+  int32_t *head = nullptr, *hscan = nullptr, *exported = nullptr, *ord = nullptr;
+  if ((rc = sc.get(&assign, C)) || (rc = sc.get(&ord, C)) || (rc = sc.get(&d.from_l2, C)) || (rc = sc.get(&keys, C)) || (rc = sc.get(&idx, C)) ||
       (rc = sc.get(&pchunk, C)) || (rc = sc.get(&order, C)) ||
       (rc = sc.get(&chunk_cnt, (int64_t)P + 1)) || (rc = sc.get(&chunk_ptr, (int64_t)P + 1)) ||
       (rc = sc.get(&ccells, C)) || (rc = sc.get(&posof, C)) ||
@@ -4764,13 +4462,21 @@ int dev_pack(mfg_ctx *ctx, DevScratch &sc, DevSweep &d) {
                            cudaMemcpyHostToDevice, st));
   MFG_CUDA(cudaMemsetAsync(chunk_cnt, 0, sizeof(int32_t) * ((size_t)P + 1), st));
   MFG_CUDA(cudaMemsetAsync(exported, 0, 4 * sizeof(int32_t), st));
+  MFG_CUDA(cudaMemsetAsync(d.from_l2, 0, C, st));
   const int32_t *cells = d.fwd ? ctx->fw_cells : ctx->bw_cells;
   const int32_t *sptr = d.fwd ? ctx->fw_sptr : ctx->bw_sptr;
   const int32_t *nbs = d.fwd ? ctx->fw_nb : ctx->bw_nb;
   const SweepRec *recs = d.fwd ? ctx->fw_recs : ctx->bw_recs;
-  k_dev_chunk_keys<<<grid_for(C), kBlock, 0, st>>>(C, cells, assign, keys, idx, chunk_cnt);
-  count_launch();
-  if ((rc = dev_sort_pairs(sc, keys, pchunk, idx, order, C, P, st))) return rc;
+  // by chunk, level, then record count (a warp's cells then have as many), by
+  // stable sorts in the reverse order
+  k_dev_count_keys<<<grid_for(C), kBlock, 0, st>>>(C, sptr, keys, idx);
+  if ((rc = dev_sort_pairs(sc, keys, pchunk, idx, order, C, 8, st))) return rc;
+  k_dev_level_keys<<<grid_for(C), kBlock, 0, st>>>(C, cells, order, d.lvl, keys);
+  if ((rc = dev_sort_pairs(sc, keys, pchunk, order, ord, C, (int32_t)d.lptr.size(), st)))
+    return rc;
+  k_dev_chunk_keys<<<grid_for(C), kBlock, 0, st>>>(C, cells, ord, assign, keys, chunk_cnt);
+  count_launch(3);
+  if ((rc = dev_sort_pairs(sc, keys, pchunk, ord, order, C, P, st))) return rc;
   if ((rc = dev_scan(sc, chunk_cnt, chunk_ptr, P + 1, st))) return rc;
   k_dev_positions<<<grid_for((int64_t)C + 1), kBlock, 0, st>>>(C, order, cells, pchunk, d.lvl,
                                                                ccells, posof, head);
@@ -4780,17 +4486,22 @@ int dev_pack(mfg_ctx *ctx, DevScratch &sc, DevSweep &d) {
   if ((rc = dev_read_i32(hscan + C, &nseg, st))) return rc;
   ChunkSweep &cs = d.fwd ? ctx->fwc : ctx->bwc;
   cs.nseg = nseg;
+  int32_t *seg_cnt = nullptr;
   if ((rc = dalloc(ctx, &cs.seg_begin, (size_t)P + 1)) ||
-      (rc = dalloc(ctx, &cs.segs, (size_t)nseg + 1)) || (rc = dalloc(ctx, &cs.cells, C)))
+      (rc = dalloc(ctx, &cs.segs, (size_t)nseg + 1)) || (rc = dalloc(ctx, &cs.cells, C)) ||
+      (rc = dalloc(ctx, &cs.seg_items, (size_t)nseg + 1)) || (rc = sc.get(&seg_cnt, (int64_t)nseg + 1)))
     return rc;
   k_dev_segs<<<grid_for((int64_t)C + 1), kBlock, 0, st>>>(C, head, hscan, cs.segs);
   k_dev_seg_begin<<<grid_for((int64_t)P + 1), kBlock, 0, st>>>(P, chunk_ptr, hscan, cs.seg_begin);
-  count_launch(2);
+  k_dev_seg_items<<<grid_for((int64_t)nseg + 1), kBlock, 0, st>>>(nseg, sweep_item_cells(W), cs.segs,
+                                                                  seg_cnt);
+  count_launch(3);
+  if ((rc = dev_scan(sc, seg_cnt, cs.seg_items, nseg + 1, st))) return rc;
   const bool mx = ctx->precision == MFG_PREC_MIXED;
   const bool with_recs = ctx->sweep_w != 0;
   const size_t nrec = with_recs ? (size_t)C * W : 0;
   const size_t nrec1 = std::max<size_t>(nrec, 1);
-  if ((rc = dalloc(ctx, &cs.nbs, nrec)) || (rc = dalloc(ctx, &cs.nslots, nrec))) return rc;
+  if ((rc = dalloc(ctx, &cs.nbs, nrec))) return rc;
   if (mx) {
     if ((rc = dalloc(ctx, &cs.recs_f, nrec))) return rc;
     MFG_CUDA(cudaMemsetAsync(cs.recs_f, 0, sizeof(SweepRecF) * nrec1, st));
@@ -4798,18 +4509,17 @@ int dev_pack(mfg_ctx *ctx, DevScratch &sc, DevSweep &d) {
     if ((rc = dalloc(ctx, &cs.recs, nrec))) return rc;
     MFG_CUDA(cudaMemsetAsync(cs.recs, 0, sizeof(SweepRec) * nrec1, st));
   }
-  MFG_CUDA(cudaMemsetAsync(cs.nbs, 0, sizeof(int32_t) * nrec1, st));
-  MFG_CUDA(cudaMemsetAsync(cs.nslots, 0, sizeof(int32_t) * nrec1, st));
+  MFG_CUDA(cudaMemsetAsync(cs.nbs, 0, sizeof(SweepNb) * nrec1, st));
   if (mx)
     k_dev_pack<true><<<grid_for(C), kBlock, 0, st>>>(
         C, W, with_recs, order, ccells, pchunk, head, hscan, cs.segs, chunk_ptr, posof, assign,
-        sptr, nbs, recs, cs.cells, cs.nbs, nullptr, cs.recs_f, cs.nslots, exported, exported + 1,
-        ctx->ring);
+        sptr, nbs, recs, cs.cells, cs.nbs, nullptr, cs.recs_f, exported, exported + 1,
+        ctx->ring, d.from_l2);
   else
     k_dev_pack<false><<<grid_for(C), kBlock, 0, st>>>(
         C, W, with_recs, order, ccells, pchunk, head, hscan, cs.segs, chunk_ptr, posof, assign,
-        sptr, nbs, recs, cs.cells, cs.nbs, cs.recs, nullptr, cs.nslots, exported, exported + 1,
-        ctx->ring);
+        sptr, nbs, recs, cs.cells, cs.nbs, cs.recs, nullptr, exported, exported + 1,
+        ctx->ring, d.from_l2);
   count_launch();
   MFG_CUDA(cudaGetLastError());
   int32_t ex[4] = {0, 0, 0, 0};
@@ -4818,6 +4528,16 @@ int dev_pack(mfg_ctx *ctx, DevScratch &sc, DevSweep &d) {
   if (d.fwd) ctx->chunk0_exported = ex[0] != 0;
   for (int k = 0; k < 3; k++) ctx->sweep_stats[d.fwd ? 0 : 1][k] = ex[1 + k];
   (d.fwd ? ctx->fw_lptr : ctx->bw_lptr) = d.lptr;
+  return MFG_OK;
+}
+
+// both sweeps packed: each arms the rows that the other reads from L2
+int dev_arm(mfg_ctx *ctx, const DevSweep &fw, const DevSweep &bw) {
+  const int32_t C = ctx->C;
+  k_dev_arm<<<grid_for(C), kBlock, 0, ctx->stream>>>(C, bw.from_l2, ctx->fwc.cells);
+  k_dev_arm<<<grid_for(C), kBlock, 0, ctx->stream>>>(C, fw.from_l2, ctx->bwc.cells);
+  count_launch(2);
+  MFG_CUDA(cudaGetLastError());
   return MFG_OK;
 }
 
@@ -4917,7 +4637,7 @@ int create_from_prep_impl(const mfg_prep_gpu *pp, const mfg_params *params, cons
     tb.join();
   }
   if ((rc = dev_pack(ctx, sc, fw))) return fail(rc);
-  if ((rc = dev_pack(ctx, sc, bw))) return fail(rc);
+  if ((rc = dev_pack(ctx, sc, bw)) || (rc = dev_arm(ctx, fw, bw))) return fail(rc);
   // node lists
   {
     int32_t *cnt = nullptr;
@@ -5375,7 +5095,7 @@ static int launch_fwd_persist(mfg_ctx *ctx, bool clamp_check, int32_t chunk_skip
   Cases cs = cases_of(ctx);
   ChunkSweep &w = ctx->fwc;
   void *recs = mx ? (void *)w.recs_f : (void *)w.recs;
-  void *args[] = {&w.seg_begin, &w.segs, &w.cells, &recs, &w.nbs, &w.nslots, (void *)&q,
+  void *args[] = {&w.seg_begin, &w.segs, &w.seg_items, &w.cells, &recs, &w.nbs, (void *)&q,
                   (void *)&qnb, &ctx->dqf, &ctx->dq8, &ctx->res, &C, &ctx->diag, &first, &P,
                   &clamp, &ctx->dt, &ctx->dt_ext, &ctx->cptr, &ctx->slots, &ctx->vol,
                   &ctx->sweep_err, &spin, &skip, &cs};
@@ -5395,16 +5115,16 @@ static int launch_bwd_persist(mfg_ctx *ctx, long long spin) {
   Cases cs = cases_of(ctx);
   ChunkSweep &w = ctx->bwc;
   void *recs = mx ? (void *)w.recs_f : (void *)w.recs;
-  void *args[] = {&w.seg_begin, &w.segs, &w.cells, &recs, &w.nbs, &w.nslots, (void *)&q,
-                  (void *)&qnb, &qn, &q4n, &ctx->dqf, &ctx->dq8, &ctx->diag, &P,
+  void *args[] = {&w.seg_begin, &w.segs, &w.seg_items, &w.cells, &recs, &w.nbs,
+                  (void *)&q, (void *)&qnb, &ctx->dqf, &ctx->dq8, &ctx->diag, &P,
                   &ctx->sweep_err, &spin, &cs};
   const void *fn = sweep_kernel(false, ctx->sweep_w, mx, ctx->ncase > 1, ctx->sweep_kind);
   if (!fn) return MFG_ERR_UNSUPPORTED;
   const int rc =
       launch_coop(fn, ctx->nchunks, sweep_threads(ctx->sweep_kind),
                   sweep_smem(ctx->sweep_w, ctx->sweep_kind), ctx->stream, args);
-  if (rc || ctx->sweep_kind != MFG_SWEEP_WIDE) return rc;
-  // the wide sweeps leave the update to a streaming pass
+  if (rc) return rc;
+  // the update, in a streaming pass
   if (mx)
     k_update_cells<true><<<grid_for(ctx->C), kBlock, 0, ctx->stream>>>(ctx->C, q, ctx->dq8, qn,
                                                                          q4n, P, cs);
@@ -5869,9 +5589,9 @@ static int rechunk(mfg_ctx *ctx, int kind, int chunking) {
     const size_t nrec = (size_t)C * W;
     dfree(cs->seg_begin, sizeof(int32_t) * ((size_t)old_chunks + 1));
     dfree(cs->segs, sizeof(int32_t) * ((size_t)cs->nseg + 1));
+    dfree(cs->seg_items, sizeof(int32_t) * ((size_t)cs->nseg + 1));
     dfree(cs->cells, sizeof(PosCell) * C);
-    dfree(cs->nbs, sizeof(int32_t) * nrec);
-    dfree(cs->nslots, sizeof(int32_t) * nrec);
+    dfree(cs->nbs, sizeof(SweepNb) * nrec);
     dfree(cs->recs, sizeof(SweepRec) * nrec);
     dfree(cs->recs_f, sizeof(SweepRecF) * nrec);
     *cs = ChunkSweep{};
@@ -5887,6 +5607,10 @@ static int rechunk(mfg_ctx *ctx, int kind, int chunking) {
     ctx->sweep_stats[k][2] = 0;
     if ((rc = dev_pack(ctx, sc, d[k]))) return rc;
   }
+  if ((rc = dev_arm(ctx, d[0], d[1]))) return rc;
+  // the rows the new tables read from L2 in the next forward sweep
+  k_arm_sentinel<<<grid_for(C), kBlock, 0, st>>>(C, ctx->dqf);
+  count_launch();
   MFG_CUDA(cudaStreamSynchronize(st));
   drop_graphs(ctx);
   return MFG_OK;

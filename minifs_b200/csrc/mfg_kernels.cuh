@@ -142,6 +142,10 @@ __device__ __forceinline__ void ldg_v8f(const float *p, float *q) {
         "=f"(q[7])
       : "l"(p));
 }
+__device__ __forceinline__ void stg_v4(double *p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d)
+               : "memory");
+}
 // load_q of an own array: the whole record
 __device__ __forceinline__ void load_q_w(const double *__restrict__ q8, int64_t c, double *q) {
   const double *p = q8 + c * Q_STRIDE;
@@ -364,36 +368,48 @@ __device__ __forceinline__ double div_recip_fast(double a, double b, double y, b
   return __fma_rn(r1, y, q1);
 }
 
-// div_recip_fast with +0 as a dividend too: its quotient steps then hold only
-// zeros, whose signs come out as the division's for either sign of b.  (The
-// sums of the sweeps start from +0 or from a residual, and a cell of no
-// records keeps them.)
-__device__ __forceinline__ double div_recip_zero(double a, double b, double y, bool &ok) {
-  const int ea = (__double2hiint(a) >> 20) & 0x7FF;
-  const int eb = (__double2hiint(b) >> 20) & 0x7FF;
-  ok = ((ea >= 523 && ea <= 1523) || __double_as_longlong(a) == 0) && eb >= 523 && eb <= 1523;
-  const double q0 = __dmul_rn(a, y);
+// The forms below report an operand outside their window through the sign of
+// an integer that is or-ed together over a cell's many divisions: a chain of
+// predicates would cost their latency each (a cell's five quotients 206 cycles
+// against 52 without them).
+__device__ __forceinline__ int hi_mag(double a) { return __double2hiint(a) & 0x7FFFFFFF; }
+// negative unless lo <= exponent of a <= hi (biased); a non-negative a's high
+// word alone orders the exponents
+__device__ __forceinline__ int outside_exp(double a, int lo, int hi) {
+  const int m = hi_mag(a);
+  return (m - (lo << 20)) | (((hi + 1) << 20) - 1 - m);
+}
+
+// RN(a / b) from y = RN(1 / b) by the steps of div_recip_fast, `near` (a
+// reciprocal within one ulp, or y) in those before the last, which only have
+// to leave the quotient faithful.  A zero a is within the window: its steps
+// give a zero, and the sign of every quotient is set to the division's.  bad
+// turns negative for an a outside [2^-500, 2^500]; b is the caller's to test.
+__device__ __forceinline__ double quot_near(double a, double b, double near, double y, int &bad) {
+  const int w = outside_exp(a, 523, 1523);
+  bad |= (hi_mag(a) | __double2loint(a)) == 0 ? 0 : w;
+  const double q0 = __dmul_rn(a, near);
   const double r0 = __fma_rn(-b, q0, a);
-  const double q1 = __fma_rn(r0, y, q0);
+  const double q1 = __fma_rn(r0, near, q0);
   const double r1 = __fma_rn(-b, q1, a);
-  return __fma_rn(r1, y, q1);
+  const double q = __fma_rn(r1, y, q1);
+  const int sign = (__double2hiint(a) ^ __double2hiint(b)) & 0x80000000;
+  return __hiloint2double((__double2hiint(q) & 0x7FFFFFFF) | sign, __double2loint(q));
 }
 
 // RN(1 / b) from an approximation y0 of it formed before b was known (the
 // sweeps': the reciprocal of the neighbour's density, b that density plus its
-// increment), for |e| <= 1/16 with e = 1 - b y0.  The geometric series 1 / b =
+// increment), for |e| < 1/16 with e = 1 - b y0.  The geometric series 1 / b =
 // y0 / (1 - e) = y0 (1 + e)(1 + e^2)(1 + e^4)(1 + O(e^8)) leaves 2^-32, a
 // Newton-Raphson step (`near`, within one ulp) and the final step of
 // rcp_rn_fast the rest: ten dependent operations instead of two conversions,
 // the hardware's approximation and six (61 against 138 cycles in one warp).
-// ok as rcp_rn_fast's, and false where e is larger.
-__device__ __forceinline__ double rcp_rn_near(double b, double y0, double &near, bool &ok) {
-  const int hb = __double2hiint(b);
-  const int eb = (hb >> 20) & 0x7FF;
+// bad turns negative where rcp_rn_fast's ok would be false or e is larger.
+__device__ __forceinline__ double rcp_rn_near(double b, double y0, double &near, int &bad) {
   const double e = __fma_rn(-b, y0, 1.0);
-  ok = eb > 1023 - 120 && eb < 1023 + 120 &&
-       !((hb & 0xFFFFF) == 0xFFFFF && (unsigned)__double2loint(b) == 0xFFFFFFFFu) &&
-       (__double2hiint(e) & 0x7FFFFFFF) < 0x3FB00000;  // |e| < 2^-4
+  const int ones = (__double2hiint(b) | 0xFFF00000) & __double2loint(b);
+  bad |= outside_exp(b, 1023 - 119, 1023 + 119) | (0x3FB00000 - 1 - hi_mag(e)) |
+         (ones == -1 ? -1 : 0);
   const double e2 = __dmul_rn(e, e);
   double y = __fma_rn(y0, e, y0);
   const double e4 = __dmul_rn(e2, e2);
@@ -403,19 +419,6 @@ __device__ __forceinline__ double rcp_rn_near(double b, double y0, double &near,
   near = __fma_rn(y, r, y);
   r = __fma_rn(-b, near, 1.0);
   return __fma_rn(near, r, near);
-}
-// div_recip_zero with `near`, a reciprocal within one ulp that is known two
-// operations earlier, in the steps before the last: they only have to leave
-// the quotient faithful.  b lies in rcp_rn_near's window.
-__device__ __forceinline__ double div_recip_near(double a, double b, double near, double y,
-                                                 bool &ok) {
-  const int ea = (__double2hiint(a) >> 20) & 0x7FF;
-  ok = (ea >= 523 && ea <= 1523) || __double_as_longlong(a) == 0;
-  const double q0 = __dmul_rn(a, near);
-  const double r0 = __fma_rn(-b, q0, a);
-  const double q1 = __fma_rn(r0, near, q0);
-  const double r1 = __fma_rn(-b, q1, a);
-  return __fma_rn(r1, y, q1);
 }
 
 // a / b for b > 0 with y = rcp_rn_fast(b): a zero a is its own quotient
@@ -499,27 +502,25 @@ __device__ __forceinline__ int rcp_seed(double rho) {
 }
 
 // flux_lusgs_fin<double> with its two divisions by Q0 as rcp_rn_near (seed:
-// rcp_seed of the neighbour's density) and div_recip_near: the same bits when
-// ok comes back true (else the caller takes the divisions).
+// rcp_seed of the neighbour's density) and quot_near: the same bits unless bad
+// turns negative (the caller then takes the divisions).
 __device__ __forceinline__ void flux_lusgs_fin_near(const LusgsPre<double> &a, int seed,
                                                     const double *DQ, double nx, double ny,
                                                     double nz, const FluxP<double> &P,
-                                                    double *flux, bool &ok) {
+                                                    double *flux, int &bad) {
   const double Q0 = a.Q0 + DQ[0];
   const double Q1 = a.Q1 + DQ[1];
   const double Q2 = a.Q2 + DQ[2];
   const double Q3 = a.Q3 + DQ[3];
   const double Q4 = a.Q4 + DQ[4];
-  bool ok0, ok1, ok2;
   double near;
-  const double y = rcp_rn_near(Q0, __hiloint2double(seed, 0), near, ok0);
-  const double rv2 = div_recip_near(0.5 * (Q1 * Q1 + Q2 * Q2 + Q3 * Q3), Q0, near, y, ok1);
+  const double y = rcp_rn_near(Q0, __hiloint2double(seed, 0), near, bad);
+  const double rv2 = quot_near(0.5 * (Q1 * Q1 + Q2 * Q2 + Q3 * Q3), Q0, near, y, bad);
   const double p = P.gamm1 * (Q4 - rv2);
   const double f0 = DQ[1] * nx + DQ[2] * ny + DQ[3] * nz;
   double v_n = a.vq;
   v_n += f0;
-  v_n = div_recip_near(v_n, Q0, near, y, ok2);
-  ok = ok0 && ok1 && ok2;
+  v_n = quot_near(v_n, Q0, near, y, bad);
   const double f1 = a.f1 + (Q1 * v_n + p * nx);
   const double f2 = a.f2 + (Q2 * v_n + p * ny);
   const double f3 = a.f3 + (Q3 * v_n + p * nz);
@@ -667,15 +668,19 @@ __device__ __forceinline__ void dq_limit_vv(const double *q, double vv, double *
   }
 }
 
-// dq_limit_vv's first test, which almost every increment passes: true where
-// the limiter scales d (T: a parameter block with the limits).
+// dq_limit_vv's first test, which almost every increment passes: negative
+// where the limiter scales d (T: a parameter block with the limits).  The
+// differences' signs are the comparisons' outcomes (a difference of unequal
+// numbers does not round to zero); one that is a NaN may only send the caller
+// to the limiter itself.
 template <typename T>
-__device__ __forceinline__ bool dq_over_limit(const double *q, double vv, const double *d,
-                                              const T &P) {
+__device__ __forceinline__ int dq_over_limit(const double *q, double vv, const double *d,
+                                             const T &P) {
   double dp = d[4] + 0.5 * d[0] * vv - (d[1] * q[1] + d[2] * q[2] + d[3] * q[3]);
   dp *= P.gamm1;
-  return (q[0] + d[0]) < P.rho_min || (q[0] + d[0]) > P.rho_max || (q[4] + dp) < P.p_min ||
-         (q[4] + dp) > P.p_max;
+  const double r = q[0] + d[0], p = q[4] + dp;
+  return __double2hiint(r - P.rho_min) | __double2hiint(P.rho_max - r) |
+         __double2hiint(p - P.p_min) | __double2hiint(P.p_max - p);
 }
 
 __device__ __forceinline__ void dq_limit(const double *q, double *d, const Params &P) {
