@@ -208,7 +208,8 @@ int mfg_set_chunking(int32_t kind);
  * permutation of 0..C-1), and the dependencies of the cell at position i
  * in nbs[sptr[i] .. sptr[i + 1]) (cell ids; ids >= C, ghosts, are not
  * dependencies).  xc, yc, zc: cell centroids [C] for the transverse
- * assignments (NULL: the vote only).  P chunks of G lane groups each;
+ * assignments (NULL: the vote only).  At most P chunks, G cells to a warp's
+ * item (16 tetrahedra);
  * force: -1 (the model's choice, as a context makes it) or MFG_CHUNK_*.
  * assign [C]: each cell's chunk; grid (optional, [2]): the transverse
  * grid Pa, Pb (a cell's chunk is la + Pa * lb), 0, 0 for the vote;
@@ -219,10 +220,11 @@ int mfg_plan_chunks(int32_t C, int32_t L, const int32_t *lptr, const int32_t *ce
                     const double *yc, const double *zc, int32_t P, int32_t G, int32_t force,
                     int32_t *assign, int32_t *grid, double *est_us);
 /* The persistent sweep kernels, in two launch shapes.  MFG_SWEEP_DEEP: one
- * block of 12 warps and one chunk per SM, the default.  MFG_SWEEP_WIDE: two
- * blocks of 6 warps and two chunks per SM.  mfg_set_sweep_kernel forces a
- * kind for contexts created afterwards (-1 restores the default).  Identical
- * results either way. */
+ * block of 12 warps and one chunk per SM.  MFG_SWEEP_WIDE: two blocks of 6
+ * warps and two chunks per SM, for widest levels of more cells per SM than
+ * its warps take at once (192 tetrahedra); a context chooses by that.
+ * mfg_set_sweep_kernel forces a kind for contexts created afterwards (-1
+ * restores the default).  Identical results either way. */
 #define MFG_SWEEP_DEEP 0
 #define MFG_SWEEP_WIDE 1
 int mfg_set_sweep_kernel(int32_t kind);

@@ -2595,11 +2595,6 @@ static size_t sweep_smem(int w, int kind) {
     return w == 8 ? sweep_smem_bytes<8, kSweepWarps / 2>() : sweep_smem_bytes<4, kSweepWarps / 2>();
   return w == 8 ? sweep_smem_bytes<8, kSweepWarps>() : sweep_smem_bytes<4, kSweepWarps>();
 }
-// Cells of a level that a kernel kind's block sweeps side by side, as the
-// chunk model counts them.
-static int32_t sweep_groups(int w, int kind) {
-  return (w == 8 ? 32 : 64) / (kind == MFG_SWEEP_WIDE ? 2 : 1);
-}
 // Cells of a warp's item in the deep sweeps.
 static int32_t sweep_item_cells(int w) {
   return w == 8 ? SweepGeom<8>::kCells : SweepGeom<4>::kCells;
@@ -3271,9 +3266,7 @@ static std::atomic<int> g_sweep_kind{-1};
 
 // Records per position (W), persistent-sweep kernel kind, grid and chunk
 // count of a new context: one chunk per resident block, no chunk under
-// kMinChunk cells.  The kind follows the widest level (max_level_cells,
-// both sweeps): where it would give a deep block more than two passes of
-// its lane groups per level, the many small blocks of the wide kernels.
+// kMinChunk cells.
 static void setup_sweep_grid(mfg_ctx *ctx, int32_t maxns, int force_kind = -1) {
   const int32_t C = ctx->C;
   ctx->sweep_w = maxns <= 4 ? 4 : (maxns <= 8 ? 8 : 0);
@@ -3283,7 +3276,15 @@ static void setup_sweep_grid(mfg_ctx *ctx, int32_t maxns, int force_kind = -1) {
     return ctx->sweep_w ? ctx->persist_occ[kind][wi] * ctx->n_sm : 0;
   };
   int kind = force_kind >= 0 ? force_kind : g_sweep_kind.load();
-  if (kind < 0) kind = MFG_SWEEP_DEEP;
+  // Two blocks per SM where the widest level has more items than the SM's
+  // warps (128^3 x 6 cells, 221 per SM and level: 1747 / 2138 us in one block,
+  // 1587 / 2002 in two); below that a chunk's level is better kept whole
+  // (104^3, 146: 813 / 1079 against 920 / 1131).
+  if (kind < 0)
+    kind = (int64_t)ctx->max_level_cells >
+                   (int64_t)kSweepWarps * sweep_item_cells(ctx->sweep_w) * std::max(1, ctx->n_sm)
+               ? MFG_SWEEP_WIDE
+               : MFG_SWEEP_DEEP;
   if (grid_of(kind) <= 0) kind = kind == MFG_SWEEP_WIDE ? MFG_SWEEP_DEEP : MFG_SWEEP_WIDE;
   ctx->sweep_kind = kind;
   ctx->persist_grid = grid_of(kind);
@@ -3389,43 +3390,57 @@ static void assign_chunks_transverse(int32_t C, int32_t Pa, int32_t Pb, int ax, 
 }
 
 // Modelled duration (SM cycles) of a persistent sweep over the chunks
-// `assign`: per level, a chunk starts after its previous level plus a
-// barrier; its k-th cell of the level waits k / G lane-group passes; a cell
-// waits for each dependency in another chunk until that one is done plus the
-// L2 round trip; a cell takes one dependent chain.  Used to choose between
-// chunk assignments.
+// `assign`: per level, a chunk starts after its previous level; its cells go
+// to items of G, whose chains run side by side but share the SM, so that each
+// item more takes kItem, and kLate more where it has to poll; a cell waits for
+// each dependency in another chunk until that one is done plus kCross, the way
+// from a store to another SM's poll.  Fitted to measured sweeps: 16^3 to 104^3
+// cubes, a tree numbering and a batch, each with the vote and a transverse
+// grid (64^3: 533 modelled, 494 us measured against 260, 269; 104^3: 1150,
+// 1158 against 800, 820).
 static double model_sweep_cycles(int32_t C, int32_t P, int32_t G,
                                  const std::vector<int32_t> &lptr, const int32_t *cells,
                                  const int32_t *sptr, const int32_t *nbs,
                                  const std::vector<int32_t> &assign) {
-  const double kChain = 800.0, kCross = 1500.0, kBarrier = 60.0;
-  std::vector<double> done(C, 0.0), tch(P, 0.0), nxt(P, 0.0);
-  std::vector<int32_t> cnt(P, 0);
+  const double kChain = 700.0, kItem = 300.0, kCross = 2700.0, kLate = 200.0;
+  struct Chunk {
+    double start = 0.0, next = 0.0;
+    int32_t count = 0, late = 0, last = -1;  // cells, late items and the last such item
+  };
+  std::vector<double> done(C, 0.0);
+  std::vector<Chunk> chunk(P);
   const int32_t L = (int32_t)lptr.size() - 1;
   double tmax = 0.0;
   for (int32_t l = 0; l < L; l++) {
     for (int32_t i = lptr[l]; i < lptr[l + 1]; i++) {
       const int32_t c = cells[i], ch = assign[c];
-      double t = tch[ch] + kBarrier + (double)(cnt[ch]++ / G) * kChain;
+      Chunk &k = chunk[ch];
+      const int32_t item = k.count++ / G;
+      const double t0 = k.start + (item + 1) * kItem + k.late * kLate;
+      double t = t0;
       for (int32_t s0 = sptr[i]; s0 < sptr[i + 1]; s0++) {
         const int32_t d = nbs[s0];
         if (d < C && assign[d] != ch) t = std::max(t, done[d] + kCross);
       }
+      if (t > t0 && k.last != item) {
+        k.last = item;
+        k.late++;
+      }
       done[c] = t + kChain;
-      nxt[ch] = std::max(nxt[ch], done[c]);
+      k.next = std::max(k.next, done[c]);
       tmax = std::max(tmax, done[c]);
     }
     for (int32_t i = lptr[l]; i < lptr[l + 1]; i++) {
-      const int32_t ch = assign[cells[i]];
-      tch[ch] = nxt[ch];
-      cnt[ch] = 0;
+      Chunk &k = chunk[assign[cells[i]]];
+      k.start = k.next;
+      k.count = k.late = 0;
+      k.last = -1;
     }
   }
   return tmax;
 }
 
-// Most cells any chunk holds on any level (more than the block's lane
-// groups take two passes over that level).
+// Most cells any chunk holds on any level.
 static int32_t max_chunk_level(int32_t P, const std::vector<int32_t> &lptr, const int32_t *cells,
                                const std::vector<int32_t> &assign) {
   std::vector<int32_t> cnt(P, 0);
@@ -3439,110 +3454,116 @@ static int32_t max_chunk_level(int32_t P, const std::vector<int32_t> &lptr, cons
 }
 
 // The chunk assignment of a sweep: the balanced vote (assign_chunks) and the
-// transverse monotone one over each pair of axes and each Pa x Pb <= P grid
-// whose aspect is within a factor two of the pair's extents.  Grids that
-// keep every level of every chunk within one pass of the lane groups come
-// first (else the fewest cells per chunk and level); among those the
-// shortest modelled sweep is kept.  Returns the choice (MFG_CHUNK_VOTE or
-// MFG_CHUNK_TRANSVERSE_*) and its modelled duration in microseconds at
-// 1.9 GHz; grid (optional) receives the transverse grid Pa, Pb (0, 0 for
-// the vote).
+// transverse monotone one over each pair of axes, the shortest modelled sweep
+// kept.  Transverse grids Pa x Pb with an aspect within a factor two of the
+// pair's extents are tried for P chunks and, where a chunk's level would hold
+// less than a warp's item and a half, for half as many, a quarter, ... (two at
+// least): fewer chunks then lengthen no level and shorten the way across them
+// (hexahedra and prisms 17^3: 53 / 56 us forward / backward over 116 chunks,
+// 46 / 48 over the model's choice; 16^3 x 6 cells: 57 / 62, 54 / 58).  On
+// grids of many cells, and with fewer chunks, only the grids nearest the
+// extents' aspect are looked at; the ones with the fewest cells per chunk and
+// level are modelled.  Returns the choice (MFG_CHUNK_VOTE or
+// MFG_CHUNK_TRANSVERSE_*) and its modelled duration in microseconds at 1.9
+// GHz; grid (optional) receives the transverse grid Pa, Pb (0, 0 for the
+// vote).
 static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int32_t> &lptr,
                          const int32_t *cells, const int32_t *sptr, const int32_t *nbs,
                          const double *const xyz[3], int force, std::vector<int32_t> &assign,
                          double *est_us, int32_t *grid = nullptr) {
-  std::vector<int32_t> best, cand;
+  std::vector<int32_t> best;
   double tbest = 1e300;
-  int32_t lbest = INT32_MAX;
   int choice = MFG_CHUNK_VOTE;
-  int32_t pa_best = 0;
+  int32_t g_best[2] = {0, 0};
   // MFG_CHUNK_TRANSVERSE_ANY: the transverse grids of every axis pair, no vote
   const bool any_t = force == MFG_CHUNK_TRANSVERSE_ANY;
   if (any_t) force = -1;
-  if ((force < 0 && !any_t) || force == MFG_CHUNK_VOTE) {
-    assign_chunks(C, P, lptr, cells, sptr, nbs, cand);
-    lbest = std::max(max_chunk_level(P, lptr, cells, cand), G);  // <= G: one pass
-    tbest = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, cand);
-    choice = MFG_CHUNK_VOTE;
-    best.swap(cand);
-  }
-  const bool geo = xyz[0] && xyz[1] && xyz[2] &&
-                   (force < 0 || force >= MFG_CHUNK_TRANSVERSE_XY);
-  if (geo) {
-    // each axis's centroid order once; the axis pairs on threads of their own
-    std::vector<int32_t> rank[3];
-    double ext[3];
-    for (int a = 0; a < 3; a++) {
-      std::vector<int32_t> idx(C);
-      for (int32_t c = 0; c < C; c++) idx[c] = c;
-      std::stable_sort(idx.begin(), idx.end(),
-                       [&](int32_t x, int32_t y) { return xyz[a][x] < xyz[a][y]; });
-      rank[a].resize(C);
-      for (int32_t r = 0; r < C; r++) rank[a][idx[r]] = r;
-      ext[a] = std::max(C ? xyz[a][idx[C - 1]] - xyz[a][idx[0]] : 0.0, 1e-300);
-    }
-    struct Best {
-      int32_t load = INT32_MAX;
-      double t = 1e300;
-      int32_t pa = 0;
-      std::vector<int32_t> assign;
-    } pb[3];
-    auto pair_search = [&](int kind) {
-      const int ax = kind == MFG_CHUNK_TRANSVERSE_YZ ? 1 : 0;
-      const int bx = kind == MFG_CHUNK_TRANSVERSE_XY ? 1 : 2;
-      Best &b = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
-      // the grids' balance first (one pass over the cells each), the model
-      // on the best-balanced three
-      std::vector<std::pair<int32_t, int32_t>> grids;  // (load, Pa)
-      std::vector<int32_t> a;
-      for (int32_t Pa = 1; Pa <= P; Pa++) {
-        const int32_t Pb = P / Pa;
-        if (Pb < 1 || (Pa > 1 && P / (Pa - 1) == Pb)) continue;  // the largest Pa per Pb
-        const double r = (double)Pa / Pb / (ext[ax] / ext[bx]);
-        if (r > 2.0 || r < 0.5) continue;
-        assign_chunks_transverse(C, Pa, Pb, ax, bx, lptr, cells, sptr, nbs, xyz, rank, a);
-        grids.push_back({std::max(max_chunk_level(P, lptr, cells, a), G), Pa});
+  const bool geo = xyz[0] && xyz[1] && xyz[2] && force != MFG_CHUNK_VOTE;
+  const bool vote = (force < 0 && !any_t) || force == MFG_CHUNK_VOTE || !geo;
+  std::vector<std::thread> th;
+  if (vote)
+    th.emplace_back([&] {
+      assign_chunks(C, P, lptr, cells, sptr, nbs, best);
+      tbest = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, best);
+    });
+  struct Best {
+    double t = 1e300;
+    int32_t pa = 0, pb = 0;
+    std::vector<int32_t> assign;
+  } pb[3];
+  std::vector<int32_t> rank[3];
+  double ext[3] = {0.0, 0.0, 0.0};
+  const bool big = C > 400000;
+  const int32_t L = std::max<int32_t>(1, (int32_t)lptr.size() - 1);
+  auto pair_search = [&](int kind) {
+    const int ax = kind == MFG_CHUNK_TRANSVERSE_YZ ? 1 : 0;
+    const int bx = kind == MFG_CHUNK_TRANSVERSE_XY ? 1 : 2;
+    Best &b = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
+    std::vector<int32_t> a;
+    for (int32_t T = P;; T /= 2) {
+      // grids of about T chunks, the largest Pa per Pb, nearest aspect first
+      std::vector<std::pair<double, std::pair<int32_t, int32_t>>> grids;
+      for (int32_t Pa = 1; Pa <= T; Pa++) {
+        const int32_t Pb = T / Pa;
+        if (Pa > 1 && Pa < T && T / (Pa + 1) == Pb) continue;
+        const double r = std::fabs(std::log((double)Pa / Pb / (ext[ax] / ext[bx])));
+        grids.push_back({r, {Pa, Pb}});
       }
       std::sort(grids.begin(), grids.end());
-      for (size_t i = 0; i < grids.size() && i < 3; i++) {
-        const int32_t load = grids[i].first, Pa = grids[i].second, Pb = P / Pa;
-        if (load > b.load) break;
+      std::vector<std::pair<int32_t, std::pair<int32_t, int32_t>>> ranked;  // (load, grid)
+      for (size_t i = 0; i < grids.size() && (i == 0 || grids[i].first < 0.7); i++) {
+        if ((big || T < P) && i >= 4) break;
+        const int32_t Pa = grids[i].second.first, Pb = grids[i].second.second;
+        assign_chunks_transverse(C, Pa, Pb, ax, bx, lptr, cells, sptr, nbs, xyz, rank, a);
+        ranked.push_back({max_chunk_level(P, lptr, cells, a), grids[i].second});
+      }
+      std::sort(ranked.begin(), ranked.end());
+      for (size_t i = 0; i < ranked.size() && i < (big || T < P ? 2 : 3); i++) {
+        const int32_t Pa = ranked[i].second.first, Pb = ranked[i].second.second;
         assign_chunks_transverse(C, Pa, Pb, ax, bx, lptr, cells, sptr, nbs, xyz, rank, a);
         const double t = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, a);
-        if (load < b.load || t < b.t) {
-          b.load = load;
+        if (t < b.t) {
           b.t = t;
           b.pa = Pa;
+          b.pb = Pb;
           b.assign.swap(a);
         }
       }
-    };
-    std::vector<std::thread> th;
+      if (T < 4 || (int64_t)C * 2 > (int64_t)3 * G * L * T) break;
+    }
+  };
+  if (geo) {
+    // each axis's centroid order, then the axis pairs, on threads of their own
+    std::vector<std::thread> tr;
+    for (int a = 0; a < 3; a++)
+      tr.emplace_back([&, a] {
+        std::vector<int32_t> idx(C);
+        for (int32_t c = 0; c < C; c++) idx[c] = c;
+        std::stable_sort(idx.begin(), idx.end(),
+                         [&](int32_t x, int32_t y) { return xyz[a][x] < xyz[a][y]; });
+        rank[a].resize(C);
+        for (int32_t r = 0; r < C; r++) rank[a][idx[r]] = r;
+        ext[a] = std::max(C ? xyz[a][idx[C - 1]] - xyz[a][idx[0]] : 0.0, 1e-300);
+      });
+    for (auto &t : tr) t.join();
     for (int kind = MFG_CHUNK_TRANSVERSE_XY; kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++)
       if (force < 0 || force == kind) th.emplace_back(pair_search, kind);
-    for (auto &t : th) t.join();
-    for (int kind = MFG_CHUNK_TRANSVERSE_XY; kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++) {
-      Best &b = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
-      if (b.assign.empty() || b.load > lbest || (b.load == lbest && b.t >= tbest)) continue;
-      lbest = b.load;
-      tbest = b.t;
-      choice = kind;
-      pa_best = b.pa;
-      best.swap(b.assign);
-    }
   }
-  if (best.empty()) {  // a forced transverse assignment without centroids
-    assign_chunks(C, P, lptr, cells, sptr, nbs, best);
-    tbest = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, best);
-    choice = MFG_CHUNK_VOTE;
-    pa_best = 0;
+  for (auto &t : th) t.join();
+  for (int kind = MFG_CHUNK_TRANSVERSE_XY; geo && kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++) {
+    Best &b = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
+    if (b.assign.empty() || b.t >= tbest) continue;
+    tbest = b.t;
+    choice = kind;
+    g_best[0] = b.pa;
+    g_best[1] = b.pb;
+    best.swap(b.assign);
   }
-  (void)lbest;
   assign.swap(best);
   if (est_us) *est_us = tbest / 1900.0;
   if (grid) {
-    grid[0] = choice == MFG_CHUNK_VOTE ? 0 : pa_best;
-    grid[1] = choice == MFG_CHUNK_VOTE ? 0 : P / pa_best;
+    grid[0] = g_best[0];
+    grid[1] = g_best[1];
   }
   return choice;
 }
@@ -3651,7 +3672,7 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
     std::vector<int32_t> assign, chunk_cnt(P, 0);
     {
       const double *xyz[3] = {m->xcc, m->ycc, m->zcc};
-      const int kind = choose_chunks(C, P, sweep_groups(ctx->sweep_w, ctx->sweep_kind), lptr,
+      const int kind = choose_chunks(C, P, sweep_item_cells(ctx->sweep_w), lptr,
                                      cells.data(),
                                      sptr.data(), nbs.data(), xyz, g_chunking.load(), assign,
                                      &ctx->chunk_est_us[fwd ? 0 : 1]);
@@ -4627,7 +4648,7 @@ int create_from_prep_impl(const mfg_prep_gpu *pp, const mfg_params *params, cons
     MFG_CUDA_OR(cudaStreamSynchronize(st));
     const double *xyz[3] = {cx.data(), cy.data(), cz.data()};
     const int force = g_chunking.load();
-    const int32_t G = sweep_groups(ctx->sweep_w, ctx->sweep_kind);
+    const int32_t G = sweep_item_cells(ctx->sweep_w);
     std::thread tb([&] {
       choose_chunks(C, P, G, bw.lptr, bw.h_cells.data(), bw.h_sptr.data(), bw.h_nbs.data(), xyz,
                     force, bw.h_assign, &ctx->chunk_est_us[1]);
@@ -5567,7 +5588,7 @@ static int rechunk(mfg_ctx *ctx, int kind, int chunking) {
     setup_sweep_grid(ctx, W, old_kind);
     return MFG_ERR_UNSUPPORTED;
   }
-  const int32_t P = ctx->nchunks, G = sweep_groups(W, ctx->sweep_kind);
+  const int32_t P = ctx->nchunks, G = sweep_item_cells(W);
   for (int k = 0; k < 2; k++) {
     const int ch = choose_chunks(C, P, G, d[k].lptr, d[k].h_cells.data(), d[k].h_sptr.data(),
                                  d[k].h_nbs.data(), xyz, chunking, d[k].h_assign,
