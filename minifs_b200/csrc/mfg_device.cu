@@ -720,8 +720,11 @@ __device__ __forceinline__ void reconstruct(double *q, int32_t c, int32_t C, int
 // the face states reconstructed to second order first (a face whose
 // reconstructed density or absolute pressure is not positive keeps its
 // first-order states).
+// Blocks of 128: a block's registers come free sooner than those of 256 threads
+// (face phase 260 -> 254 us at 64^3 x 6 cells, 970 -> 926 at 104^3).
+constexpr int kFluxBlock = 128;
 template <bool MX, bool RECON, int MINB = MFG_FLUX_MINB>
-__global__ void __launch_bounds__(kBlock, MINB)
+__global__ void __launch_bounds__(kFluxBlock, MINB * (kBlock / kFluxBlock))
 k_face_flux(int32_t F, const FaceRec *__restrict__ faces, const double *__restrict__ q8,
             Params P0, Cases cs, double *__restrict__ fflux, int32_t C, int64_t n,
             const Cen *__restrict__ fcen, const Cen *__restrict__ ccen,
@@ -1722,11 +1725,13 @@ k_update_cells(int32_t C, const double *__restrict__ q8, const double *__restric
 
 // A node's weighted sums divided by its weight (cal_gradient.cpp:2314-2324),
 // then the symmetry-plane projection of the velocity (:2330-2350).
+// acc: all five, or the first K.
+template <int K>
 __device__ __forceinline__ void node_finish(int32_t nd, int32_t info,
                                             const double *__restrict__ wnode,
-                                            const double *__restrict__ nsym, double acc[5]) {
+                                            const double *__restrict__ nsym, double acc[K]) {
   const double den = wnode[nd] + kTiny;
-  for (int v = 0; v < 5; v++) acc[v] /= den;
+  for (int v = 0; v < K; v++) acc[v] /= den;
   if (info & 2) {
     const double xs = nsym[3 * nd], ys = nsym[3 * nd + 1], zs = nsym[3 * nd + 2];
     const double un = acc[1], vn_ = acc[2], wn = acc[3];
@@ -1740,28 +1745,36 @@ __device__ __forceinline__ void node_finish(int32_t nd, int32_t info,
 // Node values of all five variables (CompNodeVar3D_dist, cal_gradient.cpp
 // :1922-2372): boundary-marked nodes average their boundary-face states,
 // the others their cells, each in the reference's accumulation order; then
-// the symmetry-plane projection of the velocity.
+// the symmetry-plane projection of the velocity.  Two lanes per node, each
+// reading one 32-byte half of every state row: the first sums rho, u, v, w,
+// the second p (its other three words go along unused).  Small grids have too
+// few nodes to hide the list's chain of loads (16^3 x 6 cells, 4913 nodes: 24
+// -> 15 us); on large ones the L1's data pipe bounds it (64^3: 84 -> 79 us,
+// halves of 16 rows per load instead of one half and a word of 32).
 __global__ void __launch_bounds__(kNodeBlock)
 k_node_values(int32_t N, int32_t C, const int32_t *__restrict__ nptr,
               const NodeEnt *__restrict__ nsl, const int32_t *__restrict__ nsptr32,
               const int32_t *__restrict__ ninfo, const double *__restrict__ wnode,
               const double *__restrict__ nsym, const int32_t *__restrict__ bface_c1,
               const double *__restrict__ q8, double *__restrict__ qn8) {
-  const int32_t nd = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nd >= N) return;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t / 2 >= N) return;
+  const int32_t nd = (int32_t)(t / 2);
+  const int h = (int)(t & 1);
   const int32_t info = ninfo[nd];
-  double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
   const int32_t ne = nptr[nd + 1] - nptr[nd];
   const NodeEnt *el = nsl + nsptr32[nd / kSlice] + nd % kSlice;  // sliced
+  const double *half = q8 + 4 * h;
   if (info & 1) {
     for (int32_t j = 0; j < ne; j++) {
       const NodeEnt en = el[(int64_t)j * kSlice];
       const int32_t k = en.src;
       const double w = en.w;
-      double qa[Q_STRIDE], qb[Q_STRIDE];
-      load_q5_w(q8, bface_c1[k], qa);
-      load_q5_w(q8, (int64_t)C + k, qb);
-      for (int v = 0; v < 5; v++) {
+      double qa[4], qb[4];
+      ldg_v4(half + (int64_t)bface_c1[k] * Q_STRIDE, qa[0], qa[1], qa[2], qa[3]);
+      ldg_v4(half + ((int64_t)C + k) * Q_STRIDE, qb[0], qb[1], qb[2], qb[3]);
+      for (int v = 0; v < 4; v++) {
         double facq = qa[v] + qb[v];
         facq *= 0.5;
         acc[v] += facq * w;
@@ -1770,19 +1783,17 @@ k_node_values(int32_t N, int32_t C, const int32_t *__restrict__ nptr,
   } else {
     for (int32_t j = 0; j < ne; j++) {
       const NodeEnt en = el[(int64_t)j * kSlice];
-      double qa[Q_STRIDE];
-      load_q5_w(q8, en.src, qa);
+      double qa[4];
+      ldg_v4(half + (int64_t)en.src * Q_STRIDE, qa[0], qa[1], qa[2], qa[3]);
       const double w = en.w;
-      for (int v = 0; v < 5; v++) acc[v] += qa[v] * w;
+      for (int v = 0; v < 4; v++) acc[v] += qa[v] * w;
     }
   }
   // a node shared with other parts of a partitioned mesh keeps its partial
   // sum until theirs are added (k_halo_nodes)
-  if (!(info & 4)) node_finish(nd, info, wnode, nsym, acc);
-  double *o = qn8 + (int64_t)nd * Q_STRIDE;
-  reinterpret_cast<double2 *>(o)[0] = make_double2(acc[0], acc[1]);
-  reinterpret_cast<double2 *>(o)[1] = make_double2(acc[2], acc[3]);
-  reinterpret_cast<double2 *>(o)[2] = make_double2(acc[4], 0.0);
+  if (!(info & 4)) node_finish<4>(nd, info, wnode, nsym, acc);
+  stg_v4(qn8 + (int64_t)nd * Q_STRIDE + 4 * h, acc[0], h ? 0.0 : acc[1], h ? 0.0 : acc[2],
+         h ? 0.0 : acc[3]);
 }
 
 // Green-Gauss face sums per cell (CompGradientQ_Gauss_Node face loops,
@@ -1828,15 +1839,15 @@ __device__ __forceinline__ void grad_faces_cell(
         for (int32_t j = j0; j < j1; j++) add(fnodes[j]);
         nn = j1 - j0;
       }
-      // the mean: a triangle's sums times RN(1/3) with Markstein's
-      // correction (the quotient's bits), else the divisions
-      const double cnt = (double)nn;
-      bool ok = nn == 3;
+      // the mean: a triangle's sums by RN(1/3) with Markstein's correction
+      // (the quotient's bits), else the divisions
+      int bad = nn == 3 ? 0 : -1;
       double t[5];
-      for (int v = 0; v < 5; v++) t[v] = quot_pos(qs[v], 3.0, kRcp3, ok);
-      if (ok) {
+      for (int v = 0; v < 5; v++) t[v] = quot_near(qs[v], 3.0, kRcp3, kRcp3, bad);
+      if (bad >= 0) {
         for (int v = 0; v < 5; v++) qs[v] = t[v];
       } else {
+        const double cnt = (double)nn;
         for (int v = 0; v < 5; v++) qs[v] /= cnt;
       }
     }
@@ -1860,14 +1871,14 @@ __device__ __forceinline__ void grad_faces_cell(
   const double vc = vol[c];
   bool ok;
   const double y = rcp_rn_fast(vc, ok);
+  int bad = ok ? 0 : -1;
   double tx[5], ty[5], tz[5];
   for (int v = 0; v < 5; v++) {
-    tx[v] = quot_pos(gx[v], vc, y, ok);
-    ty[v] = quot_pos(gy[v], vc, y, ok);
-    tz[v] = quot_pos(gz[v], vc, y, ok);
+    tx[v] = quot_near(gx[v], vc, y, y, bad);
+    ty[v] = quot_near(gy[v], vc, y, y, bad);
+    tz[v] = quot_near(gz[v], vc, y, y, bad);
   }
-  if (!(vc > 0.0)) ok = false;
-  if (!ok) {
+  if (bad < 0) {
     for (int v = 0; v < 5; v++) {
       tx[v] = gx[v] / vc;
       ty[v] = gy[v] / vc;
@@ -1895,12 +1906,13 @@ k_grad_faces(int32_t C, int64_t n, const int32_t *__restrict__ cptr,
 // Mixed form of node_finish: the sums (deviations from the freestream) times
 // the reciprocal of the weight, then the symmetry-plane projection of the
 // velocity (of value = freestream + deviation).
+template <int K>
 __device__ __forceinline__ void node_finish_mx(int32_t nd, int32_t info,
                                                const double *__restrict__ wnode,
                                                const double *__restrict__ nsym, const Params &P,
-                                               float acc[5]) {
+                                               float acc[K]) {
   const float rden = __fdividef(1.0f, (float)(wnode[nd] + kTiny));
-  for (int v = 0; v < 5; v++) acc[v] *= rden;
+  for (int v = 0; v < K; v++) acc[v] *= rden;
   if (info & 2) {
     const float xs = (float)nsym[3 * nd], ys = (float)nsym[3 * nd + 1], zs = (float)nsym[3 * nd + 2];
     const float vn = acc[1] * xs + acc[2] * ys + acc[3] * zs +
@@ -1923,39 +1935,44 @@ k_node_values_mx(int32_t N, int32_t C, const int32_t *__restrict__ nptr,
                  const int32_t *__restrict__ ninfo, const double *__restrict__ wnode,
                  const double *__restrict__ nsym, const int32_t *__restrict__ bface_c1,
                  const double *__restrict__ q8, float *__restrict__ qn4, Params P0, Cases cs) {
-  const int32_t nd = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nd >= N) return;
+  // two lanes per node, as k_node_values
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t / 2 >= N) return;
+  const int32_t nd = (int32_t)(t / 2);
+  const int h = (int)(t & 1);
   const int32_t info = ninfo[nd];
-  float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
   const int32_t ne = nptr[nd + 1] - nptr[nd];
   const NodeEnt *el = nsl + nsptr32[nd / kSlice] + nd % kSlice;  // sliced
   // the case of a node is that of any cell it touches
   const Params P = ne > 0 ? params_of(P0, cs, (info & 1) ? bface_c1[el[0].src] : el[0].src) : P0;
+  double ref[4];
+  for (int v = 0; v < 4; v++) ref[v] = h ? P.ref[4] : P.ref[v];
+  const double *half = q8 + 4 * h;
   if (info & 1) {
     for (int32_t j = 0; j < ne; j++) {
       const NodeEnt en = el[(int64_t)j * kSlice];
       const int32_t k = en.src;
       const float w = (float)en.w;
-      double qa[Q_STRIDE], qb[Q_STRIDE];
-      load_q5_w(q8, bface_c1[k], qa);
-      load_q5_w(q8, (int64_t)C + k, qb);
-      for (int v = 0; v < 5; v++)
-        acc[v] += (float)(0.5 * ((qa[v] - P.ref[v]) + (qb[v] - P.ref[v]))) * w;
+      double qa[4], qb[4];
+      ldg_v4(half + (int64_t)bface_c1[k] * Q_STRIDE, qa[0], qa[1], qa[2], qa[3]);
+      ldg_v4(half + ((int64_t)C + k) * Q_STRIDE, qb[0], qb[1], qb[2], qb[3]);
+      for (int v = 0; v < 4; v++)
+        acc[v] += (float)(0.5 * ((qa[v] - ref[v]) + (qb[v] - ref[v]))) * w;
     }
   } else {
     for (int32_t j = 0; j < ne; j++) {
       const NodeEnt en = el[(int64_t)j * kSlice];
-      double qa[Q_STRIDE];
-      load_q5_w(q8, en.src, qa);
+      double qa[4];
+      ldg_v4(half + (int64_t)en.src * Q_STRIDE, qa[0], qa[1], qa[2], qa[3]);
       const float w = (float)en.w;
-      for (int v = 0; v < 5; v++) acc[v] += (float)(qa[v] - P.ref[v]) * w;
+      for (int v = 0; v < 4; v++) acc[v] += (float)(qa[v] - ref[v]) * w;
     }
   }
   // a node shared with other parts keeps its partial sum (k_halo_nodes_mx)
-  if (!(info & 4)) node_finish_mx(nd, info, wnode, nsym, P, acc);
+  if (!(info & 4)) node_finish_mx<4>(nd, info, wnode, nsym, P, acc);
   float4 *o = reinterpret_cast<float4 *>(qn4 + (int64_t)nd * Q_STRIDE);
-  o[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-  o[1] = make_float4(acc[4], 0.f, 0.f, 0.f);
+  o[h] = h ? make_float4(acc[0], 0.f, 0.f, 0.f) : make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
 __global__ void __launch_bounds__(kGradBlockMax)
@@ -2530,7 +2547,7 @@ __global__ void k_halo_nodes(int32_t nu, const int32_t *__restrict__ unodes,
     const double *r = recv + (int64_t)eidx[e] * Q_STRIDE;
     for (int v = 0; v < 5; v++) acc[v] += r[v];
   }
-  node_finish(nd, ninfo[nd], wnode, nsym, acc);
+  node_finish<5>(nd, ninfo[nd], wnode, nsym, acc);
   for (int v = 0; v < 5; v++) o[v] = acc[v];
 }
 
@@ -2552,7 +2569,7 @@ __global__ void k_halo_nodes_mx(int32_t nu, const int32_t *__restrict__ unodes,
     const double *r = recv + (int64_t)eidx[e] * Q_STRIDE;
     for (int v = 0; v < 5; v++) acc[v] += (float)r[v];
   }
-  node_finish_mx(nd, ninfo[nd], wnode, nsym, P, acc);
+  node_finish_mx<5>(nd, ninfo[nd], wnode, nsym, P, acc);
   for (int v = 0; v < 5; v++) o[v] = acc[v];
 }
 
@@ -4956,7 +4973,7 @@ static int launch_face(mfg_ctx *ctx, bool flux, bool dtp, bool diag, double cfl,
       count_launch();
     }
 #define MFG_FLUX(MX_, R_, M_)                                                                 \
-  k_face_flux<MX_, R_, M_><<<grid_for(ctx->F), kBlock, 0, st>>>(                               \
+  k_face_flux<MX_, R_, M_><<<grid_for(ctx->F, kFluxBlock), kFluxBlock, 0, st>>>(               \
       ctx->F, ctx->faces, q, ctx->P, cs, ctx->fflux, ctx->C, ctx->n, ctx->fcen, ctx->ccen,     \
       ctx->dqdx, ctx->dqdy, ctx->dqdz, phi, ctx->halo ? ctx->h_gflag : nullptr)
     const bool fmx = mx && !ctx->flux_fp64;
@@ -5268,11 +5285,11 @@ int mfg_selftest_sweep_timeout(mfg_ctx *ctx, int64_t spin_cycles) {
 static void launch_node_values(mfg_ctx *ctx, cudaStream_t st) {
   const int nb = ctx->node_block;
   if (ctx->precision == MFG_PREC_MIXED)
-    k_node_values_mx<<<grid_for(ctx->N, nb), nb, 0, st>>>(
+    k_node_values_mx<<<grid_for(2 * (int64_t)ctx->N, nb), nb, 0, st>>>(
         ctx->N, ctx->C, ctx->nptr, ctx->nsl, ctx->nsptr32, ctx->ninfo, ctx->wnode, ctx->nsym,
         ctx->bface_c1, ctx->q8[ctx->cur], ctx->qn4, ctx->P, cases_of(ctx));
   else
-    k_node_values<<<grid_for(ctx->N, nb), nb, 0, st>>>(
+    k_node_values<<<grid_for(2 * (int64_t)ctx->N, nb), nb, 0, st>>>(
         ctx->N, ctx->C, ctx->nptr, ctx->nsl, ctx->nsptr32, ctx->ninfo, ctx->wnode, ctx->nsym,
         ctx->bface_c1, ctx->q8[ctx->cur], ctx->qn8);
   count_launch();
