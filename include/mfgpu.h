@@ -174,7 +174,7 @@ int mfg_info_get(mfg_ctx *ctx, mfg_info *info);
  * device supports cooperative launch) = one persistent kernel per sweep: the
  * LU-SGS order is cut into one contiguous chunk per resident block, a block
  * walks its chunk level by level, and a cell that depends on another chunk
- * waits, with a bounded spin, for that neighbour's ready flag.  Both modes
+ * waits, with a bounded spin, for that neighbour's increment.  Both modes
  * give identical results. */
 int mfg_set_sweep_mode(mfg_ctx *ctx, int32_t mode);
 /* Face gather and gradient face sums: lanes = 0, one thread per cell (the

@@ -421,17 +421,6 @@ __device__ __forceinline__ double rcp_rn_near(double b, double y0, double &near,
   return __fma_rn(near, r, near);
 }
 
-// a / b for b > 0 with y = rcp_rn_fast(b): a zero a is its own quotient
-// (with its sign); otherwise div_recip_fast, which clears ok outside its
-// window (the caller then divides).
-__device__ __forceinline__ double quot_pos(double a, double b, double y, bool &ok) {
-  bool okq;
-  const double q = div_recip_fast(a, b, y, okq);
-  if (a == 0.0) return a;
-  ok = ok && okq;
-  return q;
-}
-
 // FluxLUSGS3D (forward_lusgs.cpp:1271-1324) with the neighbour's sound speed
 // and conserved energy taken from its record (same expressions), in two
 // parts: what the neighbour's state and the face give, which an LU-SGS sweep
@@ -786,32 +775,6 @@ __device__ __forceinline__ int ld_relaxed(const int *p) {
 // Cycles a lane may wait for one neighbour (~2 s at 1.9 GHz) before it gives
 // up, records the failure in *err and lets the sweep run to its end.
 constexpr long long kSpinCycles = 4000000000LL;
-
-// Bounded wait for a neighbour increment produced on another SM: poll the
-// record in L2 until none of its words is the sentinel.  Returns false when
-// it gave up (or another lane did); d then holds whatever was read.
-__device__ __forceinline__ bool wait_rec(const double *rec, double *d, int *err,
-                                         long long max_cycles) {
-  load_rec5_l2(rec, d);
-  if (rec5_ready(d)) return true;
-  const long long t0 = clock64();
-  // the error word is read on every poll: polling faster (reading it every
-  // 16th poll, two polls in flight, one word per poll) or backing off with
-  // __nanosleep each measured slower on the 64^3 x 6 cube
-  int polls = 0;
-  for (;;) {
-    if (polls > 64) __nanosleep(64);
-    ++polls;
-    load_rec5_l2(rec, d);
-    const int gave_up = ld_relaxed(err);  // in flight beside the record's words
-    if (rec5_ready(d)) return true;
-    if (gave_up) return false;  // another lane gave up: finish quickly
-    if (clock64() - t0 > max_cycles) {
-      atomicExch(err, 1);
-      return false;
-    }
-  }
-}
 
 __device__ __forceinline__ void store_sentinel(double *dq8, int64_t c) {
   const double s = __longlong_as_double((long long)kSentinelBits);
