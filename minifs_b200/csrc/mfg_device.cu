@@ -3387,39 +3387,26 @@ static void assign_chunks(int32_t C, int32_t P, const std::vector<int32_t> &lptr
 // the level sets run across the two axes (the levels of a lexicographically
 // numbered box follow its slowest axis) every level spreads over all the
 // chunks.
-// rank: each cell's position in the centroid order along an axis.
+// rank: each cell's position in the centroid order along an axis; up: do the
+// dependencies lie mostly above the cell along it?
 static void assign_chunks_transverse(int32_t C, int32_t Pa, int32_t Pb, int ax, int bx,
                                      const std::vector<int32_t> &lptr, const int32_t *cells,
                                      const int32_t *sptr, const int32_t *nbs,
-                                     const double *const xyz[3],
-                                     const std::vector<int32_t> *rank,
+                                     const std::vector<int32_t> *rank, const bool *up,
                                      std::vector<int32_t> &assign) {
-  const double *ca = xyz[ax], *cb = xyz[bx];
   std::vector<int32_t> la(C), lb(C);
   for (int32_t c = 0; c < C; c++) {
     la[c] = (int32_t)((int64_t)rank[ax][c] * Pa / C);
     lb[c] = (int32_t)((int64_t)rank[bx][c] * Pb / C);
   }
   const int32_t L = (int32_t)lptr.size() - 1;
-  // per axis: do the dependencies lie mostly above (then labels take the
-  // minimum) or below the cell (the maximum)?
-  int64_t up_a = 0, up_b = 0;
   for (int32_t i = 0; i < lptr[L]; i++) {
     const int32_t c = cells[i];
     for (int32_t s0 = sptr[i]; s0 < sptr[i + 1]; s0++) {
       const int32_t d = nbs[s0];
       if (d >= C) continue;
-      up_a += (ca[d] > ca[c]) - (ca[d] < ca[c]);
-      up_b += (cb[d] > cb[c]) - (cb[d] < cb[c]);
-    }
-  }
-  for (int32_t i = 0; i < lptr[L]; i++) {
-    const int32_t c = cells[i];
-    for (int32_t s0 = sptr[i]; s0 < sptr[i + 1]; s0++) {
-      const int32_t d = nbs[s0];
-      if (d >= C) continue;
-      la[c] = up_a > 0 ? std::min(la[c], la[d]) : std::max(la[c], la[d]);
-      lb[c] = up_b > 0 ? std::min(lb[c], lb[d]) : std::max(lb[c], lb[d]);
+      la[c] = up[ax] ? std::min(la[c], la[d]) : std::max(la[c], la[d]);
+      lb[c] = up[bx] ? std::min(lb[c], lb[d]) : std::max(lb[c], lb[d]);
     }
   }
   assign.resize(C);
@@ -3434,11 +3421,12 @@ static void assign_chunks_transverse(int32_t C, int32_t Pa, int32_t Pb, int ax, 
 // from a store to another SM's poll.  Fitted to measured sweeps: 16^3 to 104^3
 // cubes, a tree numbering and a batch, each with the vote and a transverse
 // grid (64^3: 533 modelled, 494 us measured against 260, 269; 104^3: 1150,
-// 1158 against 800, 820).
+// 1158 against 800, 820).  A sweep that reaches the bound is not followed
+// further.
 static double model_sweep_cycles(int32_t C, int32_t P, int32_t G,
                                  const std::vector<int32_t> &lptr, const int32_t *cells,
                                  const int32_t *sptr, const int32_t *nbs,
-                                 const std::vector<int32_t> &assign) {
+                                 const std::vector<int32_t> &assign, double bound = 1e300) {
   const double kChain = 700.0, kItem = 300.0, kCross = 2700.0, kLate = 200.0;
   struct Chunk {
     double start = 0.0, next = 0.0;
@@ -3473,6 +3461,7 @@ static double model_sweep_cycles(int32_t C, int32_t P, int32_t G,
       k.count = k.late = 0;
       k.last = -1;
     }
+    if (tmax >= bound) break;
   }
   return tmax;
 }
@@ -3527,50 +3516,60 @@ static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int3
     double t = 1e300;
     int32_t pa = 0, pb = 0;
     std::vector<int32_t> assign;
-  } pb[3];
+  };
+  std::vector<Best> pb[3];  // of an axis pair, by the number of chunks
   std::vector<int32_t> rank[3];
+  bool up[3] = {false, false, false};
   double ext[3] = {0.0, 0.0, 0.0};
   const bool big = C > 400000;
   const int32_t L = std::max<int32_t>(1, (int32_t)lptr.size() - 1);
-  auto pair_search = [&](int kind) {
+  // grids of about T chunks over an axis pair, the largest Pa per Pb, nearest
+  // aspect first
+  auto pair_search = [&](int kind, int32_t T, Best &b) {
     const int ax = kind == MFG_CHUNK_TRANSVERSE_YZ ? 1 : 0;
     const int bx = kind == MFG_CHUNK_TRANSVERSE_XY ? 1 : 2;
-    Best &b = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
-    std::vector<int32_t> a;
-    for (int32_t T = P;; T /= 2) {
-      // grids of about T chunks, the largest Pa per Pb, nearest aspect first
-      std::vector<std::pair<double, std::pair<int32_t, int32_t>>> grids;
-      for (int32_t Pa = 1; Pa <= T; Pa++) {
-        const int32_t Pb = T / Pa;
-        if (Pa > 1 && Pa < T && T / (Pa + 1) == Pb) continue;
-        const double r = std::fabs(std::log((double)Pa / Pb / (ext[ax] / ext[bx])));
-        grids.push_back({r, {Pa, Pb}});
+    std::vector<std::pair<double, std::pair<int32_t, int32_t>>> grids;
+    for (int32_t Pa = 1; Pa <= T; Pa++) {
+      const int32_t Pb = T / Pa;
+      if (Pa > 1 && Pa < T && T / (Pa + 1) == Pb) continue;
+      const double r = std::fabs(std::log((double)Pa / Pb / (ext[ax] / ext[bx])));
+      grids.push_back({r, {Pa, Pb}});
+    }
+    std::sort(grids.begin(), grids.end());
+    struct Ranked {
+      int32_t load;
+      std::pair<int32_t, int32_t> grid;
+      std::vector<int32_t> assign;
+    };
+    const size_t keep = big || T < P ? 2 : 3;
+    std::vector<Ranked> ranked;  // the least loaded ones
+    for (size_t i = 0; i < grids.size() && (i == 0 || grids[i].first < 0.7); i++) {
+      if ((big || T < P) && i >= 4) break;
+      Ranked r;
+      r.grid = grids[i].second;
+      assign_chunks_transverse(C, r.grid.first, r.grid.second, ax, bx, lptr, cells, sptr, nbs,
+                               rank, up, r.assign);
+      r.load = max_chunk_level(P, lptr, cells, r.assign);
+      size_t at = ranked.size();
+      while (at > 0 && std::make_pair(r.load, r.grid) <
+                           std::make_pair(ranked[at - 1].load, ranked[at - 1].grid))
+        at--;
+      ranked.insert(ranked.begin() + at, std::move(r));
+      if (ranked.size() > keep) ranked.pop_back();
+    }
+    for (Ranked &r : ranked) {
+      const double t = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, r.assign, b.t);
+      if (t < b.t) {
+        b.t = t;
+        b.pa = r.grid.first;
+        b.pb = r.grid.second;
+        b.assign.swap(r.assign);
       }
-      std::sort(grids.begin(), grids.end());
-      std::vector<std::pair<int32_t, std::pair<int32_t, int32_t>>> ranked;  // (load, grid)
-      for (size_t i = 0; i < grids.size() && (i == 0 || grids[i].first < 0.7); i++) {
-        if ((big || T < P) && i >= 4) break;
-        const int32_t Pa = grids[i].second.first, Pb = grids[i].second.second;
-        assign_chunks_transverse(C, Pa, Pb, ax, bx, lptr, cells, sptr, nbs, xyz, rank, a);
-        ranked.push_back({max_chunk_level(P, lptr, cells, a), grids[i].second});
-      }
-      std::sort(ranked.begin(), ranked.end());
-      for (size_t i = 0; i < ranked.size() && i < (big || T < P ? 2 : 3); i++) {
-        const int32_t Pa = ranked[i].second.first, Pb = ranked[i].second.second;
-        assign_chunks_transverse(C, Pa, Pb, ax, bx, lptr, cells, sptr, nbs, xyz, rank, a);
-        const double t = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, a);
-        if (t < b.t) {
-          b.t = t;
-          b.pa = Pa;
-          b.pb = Pb;
-          b.assign.swap(a);
-        }
-      }
-      if (T < 4 || (int64_t)C * 2 > (int64_t)3 * G * L * T) break;
     }
   };
   if (geo) {
-    // each axis's centroid order, then the axis pairs, on threads of their own
+    // each axis's centroid order and direction, then the grids, on threads of
+    // their own
     std::vector<std::thread> tr;
     for (int a = 0; a < 3; a++)
       tr.emplace_back([&, a] {
@@ -3581,21 +3580,41 @@ static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int3
         rank[a].resize(C);
         for (int32_t r = 0; r < C; r++) rank[a][idx[r]] = r;
         ext[a] = std::max(C ? xyz[a][idx[C - 1]] - xyz[a][idx[0]] : 0.0, 1e-300);
+        const double *x = xyz[a];
+        int64_t above = 0;
+        for (int32_t i = 0; i < lptr[lptr.size() - 1]; i++)
+          for (int32_t s0 = sptr[i]; s0 < sptr[i + 1]; s0++) {
+            const int32_t c = cells[i], d = nbs[s0];
+            if (d < C) above += (x[d] > x[c]) - (x[d] < x[c]);
+          }
+        up[a] = above > 0;
       });
     for (auto &t : tr) t.join();
-    for (int kind = MFG_CHUNK_TRANSVERSE_XY; kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++)
-      if (force < 0 || force == kind) th.emplace_back(pair_search, kind);
+    std::vector<int32_t> sizes;
+    for (int32_t T = P;; T /= 2) {
+      sizes.push_back(T);
+      if (T < 4 || (int64_t)C * 2 > (int64_t)3 * G * L * T) break;
+    }
+    for (int kind = MFG_CHUNK_TRANSVERSE_XY; kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++) {
+      std::vector<Best> &of = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
+      if (force >= 0 && force != kind) continue;
+      of.resize(sizes.size());
+      for (size_t i = 0; i < sizes.size(); i++)
+        th.emplace_back([&, kind, i] { pair_search(kind, sizes[i], of[i]); });
+    }
+    for (auto &t : th) t.join();
+    th.clear();
   }
   for (auto &t : th) t.join();
-  for (int kind = MFG_CHUNK_TRANSVERSE_XY; geo && kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++) {
-    Best &b = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
-    if (b.assign.empty() || b.t >= tbest) continue;
-    tbest = b.t;
-    choice = kind;
-    g_best[0] = b.pa;
-    g_best[1] = b.pb;
-    best.swap(b.assign);
-  }
+  for (int kind = MFG_CHUNK_TRANSVERSE_XY; geo && kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++)
+    for (Best &b : pb[kind - MFG_CHUNK_TRANSVERSE_XY]) {
+      if (b.assign.empty() || b.t >= tbest) continue;
+      tbest = b.t;
+      choice = kind;
+      g_best[0] = b.pa;
+      g_best[1] = b.pb;
+      best.swap(b.assign);
+    }
   assign.swap(best);
   if (est_us) *est_us = tbest / 1900.0;
   if (grid) {
