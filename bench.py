@@ -137,7 +137,7 @@ def algorithmic_bytes(C, G, F, N, K):
         "face_gather": F * (32 + 8) + F * 24 + 40 * n + 24 * n + 8 * C + csr +
                        40 * C + 8 * C + 8 * C,
         "sweep_fwd": F * 40 + csr + 40 * n + 40 * C + 8 * C + 40 * C,
-        # backward sweep with the update fused: + the new state
+        # backward sweep and the update: + the new state
         "sweep_bwd_update": F * 40 + csr + 40 * n + 40 * C + 8 * C + 40 * C + 40 * C,
         "node_values": 40 * n + 12 * K + 8 * K + 8 * N + 40 * N,
         "grad_faces": 40 * N + F * (12 + 32 + 8) + 8 * C + 120 * n,
@@ -146,7 +146,8 @@ def algorithmic_bytes(C, G, F, N, K):
 
 
 def kernel_of_phase(phase: str, sweep_mode: int) -> str:
-    persistent = {"sweep_fwd": "k_sweep_fwd_chunk", "sweep_bwd_update": "k_sweep_bwd_chunk"}
+    persistent = {"sweep_fwd": "k_sweep_fwd_chunk",
+                  "sweep_bwd_update": "k_sweep_bwd_chunk+k_update_cells"}
     per_level = {"sweep_fwd": "k_sweep_fwd", "sweep_bwd_update": "k_sweep_bwd"}
     other = {"face_gather": "k_face_flux+k_face_gather", "node_values": "k_node_values",
              "grad_faces": "k_grad_faces", "norm": "k_norm_final"}
