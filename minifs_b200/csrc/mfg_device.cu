@@ -28,6 +28,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include <system_error>
 #include <thread>
 
 #include "mfg_internal.h"
@@ -3600,7 +3601,11 @@ static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int3
       if (force >= 0 && force != kind) continue;
       of.resize(sizes.size());
       for (size_t i = 0; i < sizes.size(); i++)
-        th.emplace_back([&, kind, i] { pair_search(kind, sizes[i], of[i]); });
+        try {
+          th.emplace_back([&, kind, i] { pair_search(kind, sizes[i], of[i]); });
+        } catch (const std::system_error &) {  // no thread to be had: here
+          pair_search(kind, sizes[i], of[i]);
+        }
     }
     for (auto &t : th) t.join();
     th.clear();
