@@ -1026,7 +1026,10 @@ k_sweep_bwd(int32_t l0, int32_t l1, const int32_t *__restrict__ cells,
 // each warp takes its items in increasing order, and every block is resident,
 // so by induction over the levels every cell completes.  Every wait is
 // bounded; one that gives up sets the error word, after which every other wait
-// returns at once and the kernel runs to its end.
+// returns at once.  A warp whose level wait gave up stops without arriving, so
+// that no barrier ever gets an arrival out of its level's turn; a poll that
+// gave up goes on in order (its results are invalid, its arrivals are not), and
+// the kernel ends either way.
 //
 // What bounds it: the dependent chain of a level -- ring read, product, sum,
 // quotient, limiter, ring write, barrier, about 900 cycles in a warp alone --
@@ -1150,20 +1153,21 @@ __device__ __forceinline__ bool mbar_test(uint64_t *b, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait for the completion of the phase of the given parity; gives up
-// (setting *err) after `spin` cycles, or soon after another wait gave up.
-// The error word and the clock are read every 64th try only.
-__device__ __forceinline__ void mbar_wait(uint64_t *b, unsigned parity, int *err,
+// Bounded wait for the completion of the phase of the given parity: false
+// when it gave up (*err is set then), after `spin` cycles or soon after
+// another wait gave up.  The error word and the clock are read every 64th try
+// only.
+__device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned parity, int *err,
                                           long long spin) {
-  if (mbar_test(b, parity)) return;
+  if (mbar_test(b, parity)) return true;
   const long long t0 = clock64();
   for (unsigned tries = 1;; tries++) {
-    if (mbar_test(b, parity)) return;
+    if (mbar_test(b, parity)) return true;
     if ((tries & 63) == 0) {
-      if (ld_relaxed(err)) return;
+      if (ld_relaxed(err)) return false;
       if (clock64() - t0 > spin) {
         atomicExch(err, 1);
-        return;
+        return false;
       }
     }
   }
@@ -1432,8 +1436,8 @@ __device__ __forceinline__ void chunk_sweep(
       FP = flux_params<typename SweepTypes<MX>::Q>(P0);
     // the read-only data of the item; a lane without a record reads its
     // cell's row instead, so that all loads are in flight together
-    // one turn, with up to N records per lane
-    auto turn = [&](auto NN) {
+    // one turn, with up to N records per lane; false when the warp has to stop
+    auto turn = [&](auto NN) -> bool {
       constexpr int N = decltype(NN)::value;
       LaneRec<MX> rec[N];
       bool has[N], far[N];
@@ -1576,14 +1580,16 @@ __device__ __forceinline__ void chunk_sweep(
           if (!__any_sync(0xffffffffu, !all)) break;
         }
       }
-      // the level before this one is in the ring
-      if (sg > 0)
-        mbar_wait(&lbar[(sg - 1) % kLevelBars], (unsigned)((sg - 1) / kLevelBars) & 1u, err, spin);
+      // the level before this one is in the ring; a wait that gave up goes the
+      // way of an operand outside the fast forms' windows, to its vote below
+      int bad = 0;
+      if (sg > 0 && !mbar_wait(&lbar[(sg - 1) % kLevelBars],
+                               (unsigned)((sg - 1) / kLevelBars) & 1u, err, spin))
+        bad = -1;
       // the dependent chain: the lanes' products, handed to the cell's first
       // lane, which sums them in record order (the other lanes go through the
       // motions), divides and tests the limiter
       double s[5], d[5], in5[5];
-      int bad = 0;
       double wf[N][5];
 #pragma unroll
       for (int u = 0; u < N; u++) {
@@ -1629,17 +1635,23 @@ __device__ __forceinline__ void chunk_sweep(
       }
       badc |= dq_over_limit(qc, vv, d, CP) & limits;
       if (h == 0 && live) bad |= badc;
-      if (__any_sync(0xffffffffu, bad < 0) && h == 0 && live) {
-        ExactArgs t;  // copies, so that the arrays above stay in registers
+      if (__any_sync(0xffffffffu, bad < 0)) {
+        // Some wait gave up: the warp stops here, its item's arrival with it.
+        // Without the level's order an arrival could reach the barrier of a
+        // level kLevelBars back that is still open and take it below zero.
+        if (__any_sync(0xffffffffu, ld_relaxed(err))) return false;
+        if (h == 0 && live) {
+          ExactArgs t;  // copies, so that the arrays above stay in registers
 #pragma unroll
-        for (int k = 0; k < 5; k++) {
-          t.in5[k] = in5[k];
-          t.qc[k] = qc[k];
+          for (int k = 0; k < 5; k++) {
+            t.in5[k] = in5[k];
+            t.qc[k] = qc[k];
+          }
+          t.P = BATCH ? *Pc : P0;
+          exact_cell<W, FWD, MX>(x.p, ns, pnb, prec, qnb, src, ring, den, limits != 0, t);
+#pragma unroll
+          for (int k = 0; k < 5; k++) d[k] = t.d[k];
         }
-        t.P = BATCH ? *Pc : P0;
-        exact_cell<W, FWD, MX>(x.p, ns, pnb, prec, qnb, src, ring, den, limits != 0, t);
-#pragma unroll
-        for (int k = 0; k < 5; k++) d[k] = t.d[k];
       }
       if (h == 0 && live) {
         double2 *rr =
@@ -1658,13 +1670,13 @@ __device__ __forceinline__ void chunk_sweep(
         stg_v4(to, h ? sn : d[0], h ? sn : d[1], h ? sn : d[2], h ? sn : d[3]);
         *reinterpret_cast<double2 *>(to + 4) = make_double2(h ? sn : d[4], 0.0);
       }
+      return true;
     };
     // most items have no lane with a second record: positions are sorted by
     // record count within a level
-    if (__any_sync(0xffffffffu, ns > L))
-      turn(std::integral_constant<int, R>());
-    else
-      turn(std::integral_constant<int, 1>());
+    const bool go = __any_sync(0xffffffffu, ns > L) ? turn(std::integral_constant<int, R>())
+                                                     : turn(std::integral_constant<int, 1>());
+    if (!go) break;
   }
   cp_async_wait<0>();
 }
