@@ -214,7 +214,9 @@ int mfg_set_chunking(int32_t kind);
  * assign [C]: each cell's chunk; grid (optional, [2]): the transverse
  * grid Pa, Pb (a cell's chunk is la + Pa * lb), 0, 0 for the vote;
  * est_us (optional): the modelled sweep duration.  Returns the assignment
- * made (MFG_CHUNK_*), MFG_ERR_INVALID for inconsistent tables. */
+ * made (MFG_CHUNK_*), MFG_ERR_INVALID for inconsistent tables,
+ * MFG_ERR_NOMEM where host memory runs out.  The search runs on up to as many
+ * threads as the host has, and on the calling one alone where none starts. */
 int mfg_plan_chunks(int32_t C, int32_t L, const int32_t *lptr, const int32_t *cells,
                     const int32_t *sptr, const int32_t *nbs, const double *xc,
                     const double *yc, const double *zc, int32_t P, int32_t G, int32_t force,

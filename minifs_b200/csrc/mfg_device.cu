@@ -18,18 +18,19 @@
 #include <atomic>
 #include <climits>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <mutex>
+#include <new>
 #include <string>
+#include <thread>
 #include <type_traits>
 #include <vector>
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
-
-#include <system_error>
-#include <thread>
 
 #include "mfg_internal.h"
 #include "mfg_kernels.cuh"
@@ -3260,6 +3261,46 @@ __global__ void k_dev_bface_c1(int32_t G, const int32_t *__restrict__ f2c,
 
 }  // namespace
 
+// Threads the host has for the chunk search.
+static int host_workers() { return std::max(1, (int)std::thread::hardware_concurrency()); }
+
+// task(0) .. task(n - 1), each once and begun in that order, on the calling
+// thread and up to workers - 1 others.  A thread that cannot be started leaves
+// its share to the rest.  What a task throws (an allocation that failed) is
+// thrown from here, once every thread has ended; the tasks not yet begun are
+// left out then.
+template <typename F>
+static void run_tasks(int n, int workers, const F &task) {
+  std::atomic<int> next{0};
+  std::mutex lock;
+  std::exception_ptr thrown;
+  auto work = [&] {
+    for (int i; (i = next.fetch_add(1)) < n;) try {
+        task(i);
+      } catch (...) {
+        next.store(n);
+        std::lock_guard<std::mutex> held(lock);
+        if (!thrown) thrown = std::current_exception();
+      }
+  };
+  {
+    struct Threads {
+      std::vector<std::thread> th;
+      ~Threads() {
+        for (auto &t : th) t.join();
+      }
+    } others;
+    try {
+      const int more = std::min(n, workers) - 1;
+      others.th.reserve(std::max(more, 0));
+      for (int k = 0; k < more; k++) others.th.emplace_back(work);
+    } catch (...) {  // none to be had: those there are, and this one
+    }
+    work();
+  }
+  if (thrown) std::rethrow_exception(thrown);
+}
+
 extern "C" {
 
 const char *mfg_error_string(int32_t code) {
@@ -3505,11 +3546,11 @@ static int32_t max_chunk_level(int32_t P, const std::vector<int32_t> &lptr, cons
 // level are modelled.  Returns the choice (MFG_CHUNK_VOTE or
 // MFG_CHUNK_TRANSVERSE_*) and its modelled duration in microseconds at 1.9
 // GHz; grid (optional) receives the transverse grid Pa, Pb (0, 0 for the
-// vote).
-static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int32_t> &lptr,
+// vote).  On up to `workers` threads.
+static int search_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int32_t> &lptr,
                          const int32_t *cells, const int32_t *sptr, const int32_t *nbs,
-                         const double *const xyz[3], int force, std::vector<int32_t> &assign,
-                         double *est_us, int32_t *grid = nullptr) {
+                         const double *const xyz[3], int force, int workers,
+                         std::vector<int32_t> &assign, double *est_us, int32_t *grid) {
   std::vector<int32_t> best;
   double tbest = 1e300;
   int choice = MFG_CHUNK_VOTE;
@@ -3519,12 +3560,6 @@ static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int3
   if (any_t) force = -1;
   const bool geo = xyz[0] && xyz[1] && xyz[2] && force != MFG_CHUNK_VOTE;
   const bool vote = (force < 0 && !any_t) || force == MFG_CHUNK_VOTE || !geo;
-  std::vector<std::thread> th;
-  if (vote)
-    th.emplace_back([&] {
-      assign_chunks(C, P, lptr, cells, sptr, nbs, best);
-      tbest = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, best);
-    });
   struct Best {
     double t = 1e300;
     int32_t pa = 0, pb = 0;
@@ -3580,49 +3615,77 @@ static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int3
       }
     }
   };
+  struct Search {
+    int kind;
+    int32_t T;
+    Best *of;
+  };
+  std::vector<Search> todo;
   if (geo) {
-    // each axis's centroid order and direction, then the grids, on threads of
-    // their own
-    std::vector<std::thread> tr;
-    for (int a = 0; a < 3; a++)
-      tr.emplace_back([&, a] {
-        std::vector<int32_t> idx(C);
-        for (int32_t c = 0; c < C; c++) idx[c] = c;
-        std::stable_sort(idx.begin(), idx.end(),
-                         [&](int32_t x, int32_t y) { return xyz[a][x] < xyz[a][y]; });
-        rank[a].resize(C);
-        for (int32_t r = 0; r < C; r++) rank[a][idx[r]] = r;
-        ext[a] = std::max(C ? xyz[a][idx[C - 1]] - xyz[a][idx[0]] : 0.0, 1e-300);
-        const double *x = xyz[a];
-        int64_t above = 0;
-        for (int32_t i = 0; i < lptr[lptr.size() - 1]; i++)
-          for (int32_t s0 = sptr[i]; s0 < sptr[i + 1]; s0++) {
-            const int32_t c = cells[i], d = nbs[s0];
-            if (d < C) above += (x[d] > x[c]) - (x[d] < x[c]);
-          }
-        up[a] = above > 0;
-      });
-    for (auto &t : tr) t.join();
     std::vector<int32_t> sizes;
     for (int32_t T = P;; T /= 2) {
       sizes.push_back(T);
       if (T < 4 || (int64_t)C * 2 > (int64_t)3 * G * L * T) break;
     }
-    for (int kind = MFG_CHUNK_TRANSVERSE_XY; kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++) {
-      std::vector<Best> &of = pb[kind - MFG_CHUNK_TRANSVERSE_XY];
-      if (force >= 0 && force != kind) continue;
-      of.resize(sizes.size());
-      for (size_t i = 0; i < sizes.size(); i++)
-        try {
-          th.emplace_back([&, kind, i] { pair_search(kind, sizes[i], of[i]); });
-        } catch (const std::system_error &) {  // no thread to be had: here
-          pair_search(kind, sizes[i], of[i]);
-        }
-    }
-    for (auto &t : th) t.join();
-    th.clear();
+    for (int kind = MFG_CHUNK_TRANSVERSE_XY; kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++)
+      if (force < 0 || force == kind) pb[kind - MFG_CHUNK_TRANSVERSE_XY].resize(sizes.size());
+    for (size_t i = 0; i < sizes.size(); i++)  // P chunks first: the most grids
+      for (int kind = MFG_CHUNK_TRANSVERSE_XY; kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++)
+        if (force < 0 || force == kind)
+          todo.push_back({kind, sizes[i], &pb[kind - MFG_CHUNK_TRANSVERSE_XY][i]});
   }
-  for (auto &t : th) t.join();
+  // an axis's centroid order and direction
+  auto axis = [&](int a) {
+    std::vector<int32_t> idx(C);
+    for (int32_t c = 0; c < C; c++) idx[c] = c;
+    std::stable_sort(idx.begin(), idx.end(),
+                     [&](int32_t x, int32_t y) { return xyz[a][x] < xyz[a][y]; });
+    rank[a].resize(C);
+    for (int32_t r = 0; r < C; r++) rank[a][idx[r]] = r;
+    ext[a] = std::max(C ? xyz[a][idx[C - 1]] - xyz[a][idx[0]] : 0.0, 1e-300);
+    const double *x = xyz[a];
+    int64_t above = 0;
+    for (int32_t i = 0; i < lptr[lptr.size() - 1]; i++)
+      for (int32_t s0 = sptr[i]; s0 < sptr[i + 1]; s0++) {
+        const int32_t c = cells[i], d = nbs[s0];
+        if (d < C) above += (x[d] > x[c]) - (x[d] < x[c]);
+      }
+    up[a] = above > 0;
+  };
+  // the axes, then the vote, then the grids, which wait for the axes: tasks
+  // begin in order, so the axes are over or on other threads by then
+  const int n_axis = geo ? 3 : 0, n_vote = vote ? 1 : 0;
+  std::mutex lock;
+  std::condition_variable axis_ended;
+  int ended = 0, sorted = 0;  // axes tried, and those that did not throw
+  run_tasks(n_axis + n_vote + (int)todo.size(), workers, [&](int i) {
+    if (i < n_axis) {
+      struct Ended {
+        std::mutex &lock;
+        std::condition_variable &cv;
+        int &n;
+        ~Ended() {
+          std::lock_guard<std::mutex> held(lock);
+          n++;
+          cv.notify_all();
+        }
+      } at_end{lock, axis_ended, ended};
+      axis(i);
+      std::lock_guard<std::mutex> held(lock);
+      sorted++;
+    } else if (i < n_axis + n_vote) {
+      assign_chunks(C, P, lptr, cells, sptr, nbs, best);
+      tbest = model_sweep_cycles(C, P, G, lptr, cells, sptr, nbs, best);
+    } else {
+      {
+        std::unique_lock<std::mutex> held(lock);
+        axis_ended.wait(held, [&] { return ended == n_axis; });
+        if (sorted < n_axis) return;
+      }
+      const Search &t = todo[i - n_axis - n_vote];
+      pair_search(t.kind, t.T, *t.of);
+    }
+  });
   for (int kind = MFG_CHUNK_TRANSVERSE_XY; geo && kind <= MFG_CHUNK_TRANSVERSE_YZ; kind++)
     for (Best &b : pb[kind - MFG_CHUNK_TRANSVERSE_XY]) {
       if (b.assign.empty() || b.t >= tbest) continue;
@@ -3639,6 +3702,18 @@ static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int3
     grid[1] = g_best[1];
   }
   return choice;
+}
+// The same, MFG_ERR_NOMEM (negative, as no choice is) where memory ran out.
+static int choose_chunks(int32_t C, int32_t P, int32_t G, const std::vector<int32_t> &lptr,
+                         const int32_t *cells, const int32_t *sptr, const int32_t *nbs,
+                         const double *const xyz[3], int force, int workers,
+                         std::vector<int32_t> &assign, double *est_us, int32_t *grid = nullptr) {
+  try {
+    return search_chunks(C, P, G, lptr, cells, sptr, nbs, xyz, force, workers, assign, est_us,
+                         grid);
+  } catch (const std::bad_alloc &) {
+    return MFG_ERR_NOMEM;
+  }
 }
 
 static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32_t> &cptr,
@@ -3747,8 +3822,9 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
       const double *xyz[3] = {m->xcc, m->ycc, m->zcc};
       const int kind = choose_chunks(C, P, sweep_item_cells(ctx->sweep_w), lptr,
                                      cells.data(),
-                                     sptr.data(), nbs.data(), xyz, g_chunking.load(), assign,
-                                     &ctx->chunk_est_us[fwd ? 0 : 1]);
+                                     sptr.data(), nbs.data(), xyz, g_chunking.load(),
+                                     host_workers(), assign, &ctx->chunk_est_us[fwd ? 0 : 1]);
+      if (kind < 0) return kind;
       if (fwd) ctx->chunking = kind;
     }
     // chunk-major, level-sorted cell lists (the level order is already sorted)
@@ -4738,13 +4814,15 @@ int create_from_prep_impl(const mfg_prep_gpu *pp, const mfg_params *params, cons
     const double *xyz[3] = {cx.data(), cy.data(), cz.data()};
     const int force = g_chunking.load();
     const int32_t G = sweep_item_cells(ctx->sweep_w);
-    std::thread tb([&] {
-      choose_chunks(C, P, G, bw.lptr, bw.h_cells.data(), bw.h_sptr.data(), bw.h_nbs.data(), xyz,
-                    force, bw.h_assign, &ctx->chunk_est_us[1]);
+    const int half = std::max(1, host_workers() / 2);
+    int kind[2] = {0, 0};
+    run_tasks(2, 2, [&](int k) {
+      DevSweep &d = k ? bw : fw;
+      kind[k] = choose_chunks(C, P, G, d.lptr, d.h_cells.data(), d.h_sptr.data(), d.h_nbs.data(),
+                              xyz, force, half, d.h_assign, &ctx->chunk_est_us[k]);
     });
-    ctx->chunking = choose_chunks(C, P, G, fw.lptr, fw.h_cells.data(), fw.h_sptr.data(),
-                                  fw.h_nbs.data(), xyz, force, fw.h_assign, &ctx->chunk_est_us[0]);
-    tb.join();
+    if (kind[0] < 0 || kind[1] < 0) return fail(std::min(kind[0], kind[1]));
+    ctx->chunking = kind[0];
   }
   if ((rc = dev_pack(ctx, sc, fw))) return fail(rc);
   if ((rc = dev_pack(ctx, sc, bw)) || (rc = dev_arm(ctx, fw, bw))) return fail(rc);
@@ -4871,7 +4949,7 @@ int mfg_set_chunking(int32_t kind) {
 int mfg_plan_chunks(int32_t C, int32_t L, const int32_t *lptr, const int32_t *cells,
                     const int32_t *sptr, const int32_t *nbs, const double *xc,
                     const double *yc, const double *zc, int32_t P, int32_t G, int32_t force,
-                    int32_t *assign, int32_t *grid, double *est_us) {
+                    int32_t *assign, int32_t *grid, double *est_us) try {
   if (C < 0 || L < 0 || P < 1 || G < 1 || !lptr || (C > 0 && (!cells || !sptr || !nbs || !assign)))
     return MFG_ERR_INVALID;
   if (force < -1 || force > MFG_CHUNK_TRANSVERSE_ANY) return MFG_ERR_INVALID;
@@ -4894,7 +4972,9 @@ int mfg_plan_chunks(int32_t C, int32_t L, const int32_t *lptr, const int32_t *ce
   std::vector<int32_t> a;
   int32_t g[2] = {0, 0};
   double us = 0.0;
-  const int choice = choose_chunks(C, P, G, lp, cells, sptr, nbs, xyz, force, a, &us, g);
+  const int choice = choose_chunks(C, P, G, lp, cells, sptr, nbs, xyz, force, host_workers(), a,
+                                   &us, g);
+  if (choice < 0) return choice;
   if (C > 0) std::copy(a.begin(), a.end(), assign);
   if (grid) {
     grid[0] = g[0];
@@ -4902,6 +4982,8 @@ int mfg_plan_chunks(int32_t C, int32_t L, const int32_t *lptr, const int32_t *ce
   }
   if (est_us) *est_us = us;
   return choice;
+} catch (const std::bad_alloc &) {
+  return MFG_ERR_NOMEM;
 }
 
 int mfg_set_sweep_kernel(int32_t kind) {
@@ -5713,12 +5795,19 @@ static int rechunk(mfg_ctx *ctx, int kind, int chunking) {
     return MFG_ERR_UNSUPPORTED;
   }
   const int32_t P = ctx->nchunks, G = sweep_item_cells(W);
+  int choice[2] = {0, 0};
+  double est[2] = {0.0, 0.0};
   for (int k = 0; k < 2; k++) {
-    const int ch = choose_chunks(C, P, G, d[k].lptr, d[k].h_cells.data(), d[k].h_sptr.data(),
-                                 d[k].h_nbs.data(), xyz, chunking, d[k].h_assign,
-                                 &ctx->chunk_est_us[k]);
-    if (k == 0) ctx->chunking = ch;
+    choice[k] = choose_chunks(C, P, G, d[k].lptr, d[k].h_cells.data(), d[k].h_sptr.data(),
+                              d[k].h_nbs.data(), xyz, chunking, host_workers(), d[k].h_assign,
+                              &est[k]);
+    if (choice[k] < 0) {  // the tables there are stay
+      setup_sweep_grid(ctx, W, old_kind);
+      return choice[k];
+    }
   }
+  ctx->chunking = choice[0];
+  for (int k = 0; k < 2; k++) ctx->chunk_est_us[k] = est[k];
   // the previous tables go; the new ones are packed as at creation
   auto dfree = [&](void *ptr, size_t bytes) {
     if (!ptr) return;
