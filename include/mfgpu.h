@@ -385,7 +385,8 @@ int mfg_iterate(mfg_ctx *ctx, int32_t n_iter, int32_t iter_done, double *norms);
  * res_out [5C] (either may be NULL).  Pinned host memory is fastest.  The
  * copies out overlap the last iteration: the residual leaves during its
  * LU-SGS sweeps, the state during its gradient (on a second stream of the
- * context); the call returns when both are in host memory. */
+ * context); the call returns when both are in host memory.  q_in has been
+ * read by then, with no outputs asked for as well. */
 int mfg_iterate_host(mfg_ctx *ctx, int32_t n_iter, int32_t iter_done, const double *q_in,
                      double *q_out, double *res_out, double *norms);
 /* Phases of one fused iteration, for mfg_profile_phases. */
@@ -525,6 +526,9 @@ int mfg_halo_phase(mfg_ctx *ctx, int32_t phase, int32_t iter_done);
 
 /* ---- data movement ----------------------------------------------------- */
 int mfg_download(mfg_ctx *ctx, int32_t field, double *host);
+/* From pinned memory the copy is still under way on return: host stays as it
+ * is until the next mfg_sync, mfg_download, mfg_iterate of one iteration or
+ * more, or (a batch) mfg_compute_timestep has returned. */
 int mfg_upload(mfg_ctx *ctx, int32_t field, const double *host);
 /* Waits for the work issued on the context's stream. */
 int mfg_sync(mfg_ctx *ctx);

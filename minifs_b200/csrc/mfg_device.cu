@@ -2742,6 +2742,7 @@ struct mfg_ctx {
   // norms coming back [hist_cap][ncase][5]; ev_tab: the table's copy is done
   double *h_tab = nullptr;
   cudaEvent_t ev_tab = nullptr;
+  bool uploading = false;  // an upload's copy may still be reading the caller's memory
   // batched cases (ncase == 1: a single grid, kernels use P)
   int32_t ncase = 1;
   std::vector<mfg_params> hps;          // per-case host parameters
@@ -5238,6 +5239,7 @@ static double cfl_for(const mfg_params &p, int32_t iter_done) {
 }
 
 static int fill_cfl_table(mfg_ctx *ctx, int32_t n_iter, int32_t iter_done);
+static int wait_upload(mfg_ctx *ctx);
 
 int mfg_compute_timestep(mfg_ctx *ctx, int32_t iter_done) {
   if (!ctx) return MFG_ERR_INVALID;
@@ -5256,6 +5258,7 @@ int mfg_compute_timestep(mfg_ctx *ctx, int32_t iter_done) {
   k_dt_clamp<<<grid_for(ctx->C), kBlock, 0, ctx->stream>>>(ctx->C, ctx->dt, ctx->dt_ext, ctx->P,
                                                            cases_of(ctx));
   count_launch();
+  if (ctx->ncase > 1 && (rc = wait_upload(ctx))) return rc;
   return check_kernel();
 }
 
@@ -5578,6 +5581,15 @@ static int fill_cfl_table(mfg_ctx *ctx, int32_t n_iter, int32_t iter_done) {
   return MFG_OK;
 }
 
+// After fill_cfl_table and the launches: the caller may change or free what it
+// uploaded before this call (from pinned memory the copy is still under way
+// when mfg_upload returns).  The table's copy follows it on the stream.
+static int wait_upload(mfg_ctx *ctx) {
+  if (ctx->uploading) MFG_CUDA(cudaEventSynchronize(ctx->ev_tab));
+  ctx->uploading = false;
+  return MFG_OK;
+}
+
 // The run's norms [n_iter][ncase][5] to pinned memory on the context's stream,
 // and from there to the caller once that stream has been waited for.
 static int fetch_norms(mfg_ctx *ctx, int32_t n_iter) {
@@ -5745,6 +5757,7 @@ int mfg_iterate(mfg_ctx *ctx, int32_t n_iter, int32_t iter_done, double *norms) 
   if (norms && (rc = fetch_norms(ctx, n_iter))) return rc;
   if ((rc = fetch_sweep_error(ctx))) return rc;
   if (norms || ctx->sweep_mode == 1) MFG_CUDA(cudaStreamSynchronize(st));
+  if ((rc = wait_upload(ctx))) return rc;
   if (norms) give_norms(ctx, n_iter, norms);
   MFG_CUDA(cudaGetLastError());
   return judge_sweep_error(ctx);
@@ -6129,6 +6142,7 @@ int mfg_iterate_host(mfg_ctx *ctx, int32_t n_iter, int32_t iter_done, const doub
   int rc;
   if (q_in && (rc = mfg_upload(ctx, MFG_FIELD_Q, q_in))) return rc;
   if (n_iter == 0 || (!q_out && !res_out)) {
+    if (n_iter == 0 && q_in) MFG_CUDA(cudaStreamSynchronize(ctx->stream));  // q_in is the caller's
     if ((rc = mfg_iterate(ctx, n_iter, iter_done, norms))) return rc;
     if (q_out && (rc = mfg_download(ctx, MFG_FIELD_Q, q_out))) return rc;
     if (res_out && (rc = mfg_download(ctx, MFG_FIELD_RES, res_out))) return rc;
@@ -6163,6 +6177,7 @@ int mfg_iterate_host(mfg_ctx *ctx, int32_t n_iter, int32_t iter_done, const doub
   if ((rc = fetch_sweep_error(ctx))) return rc;
   MFG_CUDA(cudaStreamSynchronize(st));
   MFG_CUDA(cudaStreamSynchronize(cp));
+  ctx->uploading = false;
   if (norms) give_norms(ctx, n_iter, norms);
   return judge_sweep_error(ctx);
 }
@@ -6290,6 +6305,7 @@ int mfg_upload(mfg_ctx *ctx, int32_t field, const double *host) {
   const int64_t n = ctx->n;
   MFG_CUDA(cudaMemcpyAsync(ctx->staging, host, sizeof(double) * 5 * n, cudaMemcpyHostToDevice,
                            st));
+  ctx->uploading = true;
   k_upload_q<<<grid_for(n), kBlock, 0, st>>>(ctx->staging, ctx->q8[ctx->cur],
                                             ctx->q8[ctx->cur ^ 1], ctx->q4[ctx->cur],
                                             ctx->q4[ctx->cur ^ 1], n, ctx->P, cases_of(ctx));
