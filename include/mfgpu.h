@@ -291,11 +291,14 @@ int mfg_autotune(mfg_ctx *ctx, int32_t n_trial, int32_t iter_done, int32_t flags
  * Returns MFG_ERR_TIMEOUT and leaves the context's state unchanged and
  * usable (MFG_ERR_UNSUPPORTED when the grid has a single chunk). */
 int mfg_selftest_sweep_timeout(mfg_ctx *ctx, int64_t spin_cycles);
-/* Self-test of the sweeps' division by a precomputed reciprocal (no
+/* Self-test of the division by a precomputed reciprocal, as the sweeps
+ * divide by the diagonal and the gradient by a triangle's node count (no
  * counterpart in the reference): n pseudo-random dividend/divisor pairs
- * (seeded, exponents across [-600, 600]) divided both ways on the current
- * device; *mismatches receives the number of results whose bits differ
- * from the division's (0 expected). */
+ * (seeded, exponents across [-600, 600]; zero, subnormal and non-finite
+ * dividends among them) divided both ways on the current device; *mismatches
+ * receives the number of quotients whose bits differ from the division's,
+ * that are left to the division inside [2^-500, 2^501), or that are taken
+ * outside it (0 expected). */
 int mfg_selftest_division(int64_t n, uint64_t seed, int64_t *mismatches);
 /* Known-answer self-test of the device arithmetic (test hook; the inputs
  * are the reference functions' own arguments): runs the device functions

@@ -2318,11 +2318,14 @@ __global__ void k_norm_seg_final(int32_t nparts, const double *__restrict__ part
 
 __global__ void k_counter_inc(int32_t *__restrict__ counter) { *counter += 1; }
 
-// Self-test of div_by_recip against the division: n dividend/divisor pairs
-// from a splitmix64 stream, significands uniform, exponents uniform in
-// [-600, 600] (both sides of div_by_recip's window) and random signs; every
-// fourth divisor has an all-ones significand.  Counts the pairs whose bits
-// differ.
+// Self-test of quot_near against the division, in the forms of the sweeps'
+// diagonal (a reciprocal that was divided for) and of a triangle's mean: n
+// dividend/divisor pairs from a splitmix64 stream, significands uniform,
+// exponents uniform in [-600, 600] (both sides of the window) and random
+// signs; every fourth divisor has an all-ones significand, three in 32
+// dividends are a zero, a subnormal, and an infinity or a NaN.  Counts the
+// quotients whose bits differ, and those left to the division inside the
+// window or taken outside it.
 __device__ __forceinline__ uint64_t splitmix64(uint64_t &x) {
   uint64_t z = (x += 0x9E3779B97F4A7C15ull);
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -2343,11 +2346,29 @@ __global__ void k_selftest_division(int64_t n, uint64_t seed,
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     uint64_t x = seed ^ ((uint64_t)i * 0xD1B54A32D192ED03ull);
-    const double a = draw_double(x, false);
+    double a = draw_double(x, false);
     const double b = draw_double(x, (i & 3) == 3);
-    const double y = 1.0 / b;
-    const double q = div_by_recip(a, b, y), ref = a / b;
-    if (__double_as_longlong(q) != __double_as_longlong(ref)) local++;
+    const int odd = (int)(i >> 2) & 31;  // of divisors of both kinds
+    if (odd < 3) {
+      const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+      const unsigned long long keep =
+          odd == 0 ? 0 : odd == 1 ? 0xFFFFFFFFFFFFFull : (u & 1 ? 0xFFFFFFFFFFFFFull : 0);
+      a = __longlong_as_double((long long)((u & (0x8000000000000000ull | keep)) |
+                                           (odd == 2 ? 0x7FF0000000000000ull : 0)));
+    }
+    auto inside = [](double v) {
+      const int e = (__double2hiint(v) >> 20) & 0x7FF;
+      return e >= 1023 - 500 && e <= 1023 + 500;
+    };
+    auto check = [&](double by, double y, int bad) {
+      const double q = quot_near(a, by, y, y, bad);
+      if ((bad >= 0) != ((a == 0.0 || inside(a)) && inside(by)))
+        local++;
+      else if (bad >= 0 && __double_as_longlong(q) != __double_as_longlong(a / by))
+        local++;
+    };
+    check(b, 1.0 / b, outside_exp(b, 523, 1523));
+    check(3.0, kRcp3, 0);
   }
   if (local) atomicAdd(bad, local);
 }
@@ -2433,9 +2454,9 @@ __global__ void k_selftest_division_fast(int64_t n, uint64_t seed,
       continue;
     }
     if (__double_as_longlong(y) != __double_as_longlong(1.0 / b)) b0++;
-    bool okq;
-    const double q = div_recip_fast(a, b, y, okq);
-    if (okq && __double_as_longlong(q) != __double_as_longlong(a / b)) b1++;
+    int bady = 0;  // the gradient's form, by a volume
+    const double q = quot_near(a, b, y, y, bady);
+    if (bady < 0 || __double_as_longlong(q) != __double_as_longlong(a / b)) b1++;
     // from the seed of a divisor within 1/16 of b
     const double b0f = b * (1.0 + ((double)(int64_t)(ra >> 12) * 0x1p-52 - 0.5) * 0.115);
     double near;
@@ -2446,7 +2467,7 @@ __global__ void k_selftest_division_fast(int64_t n, uint64_t seed,
     } else {
       if (__double_as_longlong(yn) != __double_as_longlong(1.0 / b)) b0++;
       const double qn = quot_near(a, b, near, yn, badq);
-      if (badq >= 0 && __double_as_longlong(qn) != __double_as_longlong(a / b)) b1++;
+      if (badq < 0 || __double_as_longlong(qn) != __double_as_longlong(a / b)) b1++;
       const double z = copysign(0.0, a), qz = quot_near(z, b, near, yn, badz);
       if (badz < 0 || __double_as_longlong(qz) != __double_as_longlong(z / b)) b1++;
     }

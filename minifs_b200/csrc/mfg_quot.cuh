@@ -1,0 +1,71 @@
+// Quotients without a division, to the division's bits.  Nothing but integer
+// and floating-point operations on doubles (tests/quotient_check.cpp compiles
+// this file for the host).
+#pragma once
+
+namespace mfg {
+
+// The forms below report an operand outside their window through the sign of
+// an integer that is or-ed together over a cell's many divisions: a chain of
+// predicates would cost their latency each (a cell's five quotients 206 cycles
+// against 52 without them).
+__device__ __forceinline__ int hi_mag(double a) { return __double2hiint(a) & 0x7FFFFFFF; }
+// negative unless lo <= exponent of a <= hi (biased); a non-negative a's high
+// word alone orders the exponents
+__device__ __forceinline__ int outside_exp(double a, int lo, int hi) {
+  const int m = hi_mag(a);
+  return (m - (lo << 20)) | (((hi + 1) << 20) - 1 - m);
+}
+
+// Correctly rounded a / b from y = RN(1 / b), for a divisor known before the
+// dividend (the LU-SGS diagonal, a cell's volume, a triangle's three nodes):
+// the quotient's dependent chain is one product and four fused multiply-adds
+// instead of a division.  Markstein's theorem (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34(1), 1990): for y within half an ulp of 1/b and q within one ulp of
+// a/b, r = a - b q is exact and RN(q + r y) = RN(a / b).  q0 = RN(a near) is
+// within two ulps; one correction step makes it faithful, the second rounds
+// correctly.  `near` (a reciprocal within one ulp, or y) serves in the steps
+// before the last.  A zero a is within the window: its steps give a zero, and
+// the sign of every quotient is set to the division's.  bad turns negative for
+// an a that is neither zero nor of an exponent in [-500, 500] (subnormals,
+// overflow risks, non-finite values); b is the caller's to test, with the same
+// bounds.  The caller then takes the division itself.
+__device__ __forceinline__ double quot_near(double a, double b, double near, double y, int &bad) {
+  const int w = outside_exp(a, 523, 1523);
+  bad |= (hi_mag(a) | __double2loint(a)) == 0 ? 0 : w;
+  const double q0 = __dmul_rn(a, near);
+  const double r0 = __fma_rn(-b, q0, a);
+  const double q1 = __fma_rn(r0, near, q0);
+  const double r1 = __fma_rn(-b, q1, a);
+  const double q = __fma_rn(r1, y, q1);
+  const int sign = (__double2hiint(a) ^ __double2hiint(b)) & 0x80000000;
+  return __hiloint2double((__double2hiint(q) & 0x7FFFFFFF) | sign, __double2loint(q));
+}
+
+// RN(1 / b) from an approximation y0 of it formed before b was known (the
+// sweeps': the reciprocal of the neighbour's density, b that density plus its
+// increment), for |e| < 1/16 with e = 1 - b y0.  The geometric series 1 / b =
+// y0 / (1 - e) = y0 (1 + e)(1 + e^2)(1 + e^4)(1 + O(e^8)) leaves 2^-32, a
+// Newton-Raphson step (`near`, within one ulp) and the final step of
+// rcp_rn_fast the rest: ten dependent operations instead of two conversions,
+// the hardware's approximation and six (61 against 138 cycles in one warp).
+// bad turns negative outside exponents of [-119, 119], for an all-ones
+// significand (as rcp_rn_fast's ok) and where e is larger.
+__device__ __forceinline__ double rcp_rn_near(double b, double y0, double &near, int &bad) {
+  const double e = __fma_rn(-b, y0, 1.0);
+  const int ones = (__double2hiint(b) | 0xFFF00000) & __double2loint(b);
+  bad |= outside_exp(b, 1023 - 119, 1023 + 119) | (0x3FB00000 - 1 - hi_mag(e)) |
+         (ones == -1 ? -1 : 0);
+  const double e2 = __dmul_rn(e, e);
+  double y = __fma_rn(y0, e, y0);
+  const double e4 = __dmul_rn(e2, e2);
+  y = __fma_rn(y, e2, y);
+  y = __fma_rn(y, e4, y);
+  double r = __fma_rn(-b, y, 1.0);
+  near = __fma_rn(y, r, y);
+  r = __fma_rn(-b, near, 1.0);
+  return __fma_rn(near, r, near);
+}
+
+}  // namespace mfg
