@@ -20,6 +20,7 @@
 #include <cmath>
 #include <condition_variable>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <exception>
 #include <mutex>
@@ -2759,9 +2760,11 @@ struct mfg_ctx {
   double *norm_part = nullptr, *norm_out = nullptr, *norm_hist = nullptr, *cfl_tab = nullptr;
   int32_t *iter_counter = nullptr;
   int32_t hist_cap = 0;
-  // pinned: the CFL table of the run being launched [hist_cap][ncase], the
-  // norms coming back [hist_cap][ncase][5]; ev_tab: the table's copy is done
+  // pinned (pageable where no pinned memory is to be had): the CFL table of the
+  // run being launched [hist_cap][ncase], the norms coming back
+  // [hist_cap][ncase][5]; ev_tab: the table's copy is done
   double *h_tab = nullptr;
+  bool h_tab_pinned = false;
   cudaEvent_t ev_tab = nullptr;
   bool uploading = false;  // an upload's copy may still be reading the caller's memory
   // batched cases (ncase == 1: a single grid, kernels use P)
@@ -3345,6 +3348,15 @@ const char *mfg_last_cuda_error(void) { return g_cuda_error.c_str(); }
 
 int64_t mfg_kernel_launches(void) { return g_launches.load(); }
 
+static void free_tab(mfg_ctx *ctx) {
+  if (ctx->h_tab_pinned)
+    cudaFreeHost(ctx->h_tab);
+  else
+    std::free(ctx->h_tab);
+  ctx->h_tab = nullptr;
+  ctx->h_tab_pinned = false;
+}
+
 static void free_ctx(mfg_ctx *ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
@@ -3352,7 +3364,7 @@ static void free_ctx(mfg_ctx *ctx) {
     if (ctx->graph[k]) cudaGraphExecDestroy(ctx->graph[k]);
   for (void *p : ctx->allocs) cudaFree(p);
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
-  if (ctx->h_tab) cudaFreeHost(ctx->h_tab);
+  free_tab(ctx);
   if (ctx->ev_tab) cudaEventDestroy(ctx->ev_tab);
   if (ctx->ev_res) cudaEventDestroy(ctx->ev_res);
   if (ctx->ev_state) cudaEventDestroy(ctx->ev_state);
@@ -5569,13 +5581,16 @@ static int ensure_tables(mfg_ctx *ctx, int32_t n_iter) {
   if (ctx->h_tab) {
     MFG_CUDA(cudaEventSynchronize(ctx->ev_tab));
     MFG_CUDA(cudaStreamSynchronize(ctx->stream));
-    cudaFreeHost(ctx->h_tab);
-    ctx->h_tab = nullptr;
+    free_tab(ctx);
     ctx->hist_cap = 0;
   }
   if (!ctx->ev_tab) MFG_CUDA(cudaEventCreateWithFlags(&ctx->ev_tab, cudaEventDisableTiming));
-  if (cudaMallocHost((void **)&ctx->h_tab, sizeof(double) * 6 * cap * ctx->ncase) != cudaSuccess)
-    return MFG_ERR_NOMEM;
+  const size_t bytes = sizeof(double) * 6 * cap * ctx->ncase;
+  ctx->h_tab_pinned = cudaMallocHost((void **)&ctx->h_tab, bytes) == cudaSuccess;
+  if (!ctx->h_tab_pinned) {  // the copies are slower from there, no more
+    cudaGetLastError();
+    if (!(ctx->h_tab = (double *)std::malloc(bytes))) return MFG_ERR_NOMEM;
+  }
   ctx->hist_cap = cap;
   return MFG_OK;
 }
