@@ -116,7 +116,7 @@ typedef struct mfg_info {
   int32_t sweep_chunking;           /* persistent sweeps: chunk assignment (MFG_CHUNK_*) */
   /* records of the [forward, backward] sweep whose neighbour increment is
    * read from the block's shared-memory ring, from global memory (same
-   * chunk, older than the ring) and from another chunk (polled in L2) */
+   * chunk, not in the ring) and from another chunk (polled in L2) */
   int32_t sweep_ring_records[2], sweep_global_records[2], sweep_cross_records[2];
   double sweep_model_us[2];         /* modelled duration of each sweep with its chunks */
   int32_t sweep_kernel;             /* persistent sweep kernels (MFG_SWEEP_*) */

@@ -1020,8 +1020,8 @@ k_sweep_bwd(int32_t l0, int32_t l1, const int32_t *__restrict__ cells,
 // the phase is never mistaken for another's.
 //
 // A dependency inside the chunk is read from the block's shared-memory ring
-// of its last kRing positions.  One in another chunk, or older than the ring,
-// comes from L2: it is copied into a row of the lane's own while the item's
+// of its last kRing positions (in_ring).  One in another chunk, or not in the
+// ring, comes from L2: it is copied into a row of the lane's own while the item's
 // other data are read, and polled (bounded) while it is still the sentinel.
 // Only the rows that some record reads from L2 are armed with the sentinel
 // (PosCell's kArm).  Progress: a cell waits only for cells of lower levels,
@@ -1059,6 +1059,15 @@ constexpr int kMinChunk = 64;              // no chunk smaller than this many ce
 #endif
 constexpr int kRing = MFG_SWEEP_RING;
 static_assert((kRing & (kRing - 1)) == 0, "ring size must be a power of two");
+// Whether the ring holds the increment of the cell at position p, whose level
+// starts at position p_level of the chunk, when the level that ends at
+// position end reads it.  Positions a multiple of ring apart share a row.  A
+// later one must belong to a later level than the reader's.  An earlier one
+// must not belong to the cell's own level: a level's items are taken by
+// different warps, in no order among themselves, so it could write last.
+__host__ __device__ inline bool in_ring(int32_t p, int32_t p_level, int32_t end, int32_t ring) {
+  return p >= end - ring && p < p_level + ring;
+}
 
 // Warps per SM, in one block (MFG_SWEEP_DEEP) or two (MFG_SWEEP_WIDE).
 constexpr int kSweepWarps = 12;
@@ -1475,7 +1484,7 @@ __device__ __forceinline__ void chunk_sweep(
       };
 #pragma unroll
       for (int u = 0; u < N; u++) load_rec(u);
-      // increments that come from L2 (older than the ring, or another chunk's):
+      // increments that come from L2 (not in the ring, or another chunk's):
       // copied into the lane's rows while the rest is read and formed
       int row[N];
       bool l2 = false;
@@ -2752,7 +2761,7 @@ struct mfg_ctx {
   int chunking = 0;              // chunk assignment of the forward sweep (MFG_CHUNK_*)
   double chunk_est_us[2] = {0.0, 0.0};  // modelled duration of each sweep with its chunks
   // records of each sweep [forward, backward] whose increment comes from the
-  // block's ring, from global memory (same chunk, older than the ring), or
+  // block's ring, from global memory (same chunk, not in the ring), or
   // from another chunk
   int32_t sweep_stats[2][3] = {{0, 0, 0}, {0, 0, 0}};
   int n_sm = 0;
@@ -3173,7 +3182,8 @@ __global__ void k_dev_pack(int32_t C, int32_t W, int with_recs, const int32_t *_
     if (cross) {
       e |= kMark;
       atomicAdd(&stats[2], 1);
-    } else if (nb < C && posof[nb] >= seg_end - ring) {
+    } else if (nb < C && in_ring(posof[nb], segs[hscan[posof[nb]] + head[posof[nb]] - 1],
+                                 seg_end, ring)) {
       e |= kInRing;
       slot = (posof[nb] - chunk_ptr[p]) & (ring - 1);
       atomicAdd(&stats[0], 1);
@@ -3882,7 +3892,7 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
     // position-major: the records of position k at [k * W, k * W + ns)
     std::vector<SweepNb> cnbs((size_t)C * W, SweepNb{0, 0});
     std::vector<SweepRec> crecs((size_t)C * W, SweepRec{0.0, 0.0, 0.0, 0.0});
-    std::vector<int32_t> posof(C);
+    std::vector<int32_t> posof(C), level_start(C);  // of each cell's level in its chunk
     for (int32_t k = 0; k < C; k++) posof[ccells[k]] = k;
     std::vector<PosCell> &packed = packed_of[fwd ? 0 : 1];
     packed.resize(C);
@@ -3897,6 +3907,7 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
           seg_end = k;
           while (seg_end < chunk_ptr[p + 1] && lv[ccells[seg_end]] == lv[c]) seg_end++;
         }
+        level_start[c] = segs.back();
         const int32_t gi = gpos[c];
         packed[k] = PosCell{c, sptr[gi + 1] - sptr[gi]};
         if (!ctx->sweep_w) continue;  // no persistent sweeps for this grid
@@ -3907,18 +3918,18 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
           if (cross && assign[nb] == 0) chunk0_exported = true;
           uint32_t e = (uint32_t)nb;
           int32_t *stat = ctx->sweep_stats[fwd ? 0 : 1];
-          if (nb < C && (cross || posof[nb] < seg_end - ctx->ring)) from_l2[fwd ? 0 : 1][nb] = 1;
+          const bool ring = nb < C && !cross &&
+                            in_ring(posof[nb], level_start[nb], seg_end, ctx->ring);
+          if (nb < C && !ring) from_l2[fwd ? 0 : 1][nb] = 1;
           if (cross) {
             e |= kMark;
             stat[2]++;
-          } else if (nb < C && posof[nb] >= seg_end - ctx->ring) {
-            // still in the ring when this level reads it: overwritten only by
-            // position posof[nb] + ring, which lies in a later level
+          } else if (ring) {
             e |= kInRing;
             cnbs[o].slot = (posof[nb] - chunk_ptr[p]) & (ctx->ring - 1);
             stat[0]++;
           } else if (nb < C) {
-            stat[1]++;  // in the chunk, older than the ring: read from global memory
+            stat[1]++;  // in the chunk, not in the ring: read from global memory
           }
           cnbs[o].nb = e;
           crecs[o] = recs[s0];
