@@ -111,7 +111,7 @@ typedef struct mfg_info {
   int32_t graph_ready;
   int32_t ncase;                    /* independent cases in the context (1 unless batched) */
   int32_t sweep_chunks;             /* persistent sweeps: chunks (= resident blocks) */
-  int32_t sweep_lanes;              /* persistent sweeps: lanes per cell */
+  int32_t sweep_lanes;              /* persistent sweeps: mfg_set_sweep_lanes' value */
   int32_t sweep_records;            /* persistent sweeps: record slots per cell (4 or 8) */
   int32_t sweep_chunking;           /* persistent sweeps: chunk assignment (MFG_CHUNK_*) */
   /* records of the [forward, backward] sweep whose neighbour increment is
@@ -174,8 +174,9 @@ int mfg_info_get(mfg_ctx *ctx, mfg_info *info);
  * device supports cooperative launch) = one persistent kernel per sweep: the
  * LU-SGS order is cut into one contiguous chunk per resident block, a block
  * walks its chunk level by level, and a cell that depends on another chunk
- * waits, with a bounded spin, for that neighbour's increment.  Both modes
- * give identical results. */
+ * waits, with a bounded spin, for that neighbour's increment.  Contexts whose
+ * cells have more than 8 lower or upper neighbours, and batches of more than
+ * 2^22 cases, have 0 only.  Both modes give identical results. */
 int mfg_set_sweep_mode(mfg_ctx *ctx, int32_t mode);
 /* Face gather and gradient face sums: lanes = 0, one thread per cell (the
  * default), or one lane per face of a cell with the per-cell sums passed
@@ -183,8 +184,9 @@ int mfg_set_sweep_mode(mfg_ctx *ctx, int32_t mode);
  * at most 4 faces, 8 where at most 8; other values MFG_ERR_UNSUPPORTED).
  * Identical results, norms included; the autotuner times both. */
 int mfg_set_gather_lanes(mfg_ctx *ctx, int32_t lanes);
-/* Persistent sweeps: lanes per cell; the record slots per cell W is the
- * only value the current kernels take (others: MFG_ERR_UNSUPPORTED). */
+/* Persistent sweeps: kept for callers of earlier kernels, whose lanes per
+ * cell it chose.  The record slots per cell W is the only value taken
+ * (others: MFG_ERR_UNSUPPORTED) and changes nothing: a cell has W / 2 lanes. */
 int mfg_set_sweep_lanes(mfg_ctx *ctx, int32_t lanes);
 /* Chunk assignments of the persistent sweeps (one chunk per block).
  * MFG_CHUNK_VOTE: level by level a cell joins the chunk most of its
@@ -230,11 +232,9 @@ int mfg_plan_chunks(int32_t C, int32_t L, const int32_t *lptr, const int32_t *ce
 #define MFG_SWEEP_DEEP 0
 #define MFG_SWEEP_WIDE 1
 int mfg_set_sweep_kernel(int32_t kind);
-/* Times n_trial fused iterations with each lane count the persistent
- * sweeps take on this context's own grid and keeps the faster (ms_out[2],
- * optional, receives the ms per iteration of W and W / 2 lanes; the
- * current kernels take W only, so ms_out[1] is -1).  mfg_autotune covers
- * this and the other launch parameters.  The state and the dt extrema are
+/* Times n_trial fused iterations with the one value mfg_set_sweep_lanes
+ * takes on this context's own grid (ms_out[2], optional, receives the ms per
+ * iteration and -1).  mfg_autotune times the other launch parameters.  The state and the dt extrema are
  * restored afterwards; res, dt, Diag, DQ and the gradient hold the last
  * trial iteration's values.  iter_done: the CFL ramp position to time at. */
 int mfg_autotune_sweeps(mfg_ctx *ctx, int32_t n_trial, int32_t iter_done, double *ms_out);
@@ -287,7 +287,8 @@ int mfg_autotune(mfg_ctx *ctx, int32_t n_trial, int32_t iter_done, int32_t flags
                  mfg_tune_report *rep);
 /* Failure-detection self-test of the bounded waits: runs a forward sweep
  * whose first chunk is withheld, so the cells that depend on it wait for
- * flags that are never set; each wait gives up after spin_cycles SM cycles.
+ * increments that are never written; each wait gives up after spin_cycles SM
+ * cycles, and a warp whose wait for a level gave up stops there.
  * Returns MFG_ERR_TIMEOUT and leaves the context's state unchanged and
  * usable (MFG_ERR_UNSUPPORTED when the grid has a single chunk). */
 int mfg_selftest_sweep_timeout(mfg_ctx *ctx, int64_t spin_cycles);

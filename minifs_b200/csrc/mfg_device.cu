@@ -1042,13 +1042,12 @@ k_sweep_bwd(int32_t l0, int32_t l1, const int32_t *__restrict__ cells,
 // memory for lane pairs of other warps, update by the producers; then whole
 // items per warp with the update in the sweep, a sentinel for every row, the
 // L2 increments polled before the level's wait and one level search per
-// level): 64^3 x 6 cells 511 / 565, 334 / 396, now 270 / 322; 128^3 3057 /
-// 3157 (blocks of two warps), -, 1758 / 2147; 16^3 117 / 132, 63 / 64, 57 /
-// 62.  Measured and not kept: thread-per-cell items (353 / 429), 14 or 16
+// level): 64^3 x 6 cells 511 / 565, 334 / 396, now 266 / 321; 128^3 3057 /
+// 3157 (blocks of two warps), -, 1577 / 2005; 16^3 117 / 132, 63 / 64, 52 /
+// 58.  Measured and not kept: thread-per-cell items (353 / 429), 14 or 16
 // warps of 128 registers (spills; 362 / 408), the item's rows by cp.async a
 // turn ahead (317 / 375: their shared-memory round trip loads the data pipe).
 // ---------------------------------------------------------------------------
-constexpr uint32_t kMark = 0x80000000u;    // neighbour flag: in another chunk (wait in L2)
 constexpr uint32_t kInRing = 0x40000000u;  // neighbour flag: increment in the block's ring
 constexpr uint32_t kIdMask = 0x3FFFFFFFu;  // neighbour id bits
 constexpr int kMinChunk = 64;              // no chunk smaller than this many cells
@@ -1096,7 +1095,7 @@ struct __align__(8) PosCell {
 constexpr int kArm = 256;
 constexpr int kCaseShift = 9;
 constexpr int32_t kMaxSweepCases = 1 << (31 - kCaseShift);
-// A record's neighbour (flags kMark / kInRing) and, in the ring, its row.
+// A record's neighbour (flag kInRing) and, in the ring, its row.
 struct __align__(8) SweepNb {
   uint32_t nb;
   int32_t slot;
@@ -1336,7 +1335,7 @@ constexpr size_t sweep_smem_bytes() {
 // One persistent sweep over chunk blockIdx.x (see the section comment).  FWD:
 // DQ* = (res - sum_j 0.5 area_j F_j) / Diag, limited except for the first
 // cell (SolveLUSGS3D forward, forward_lusgs.cpp:803-1014); backward: DQ = DQ*
-// - (sum_j area_j F_j) / (2 Diag), limited (:1060-1249), then the update.
+// - (sum_j area_j F_j) / (2 Diag), limited (:1060-1249); the update is k_update_cells'.
 template <int W, bool FWD, bool MX, bool BATCH, int NW>
 __device__ __forceinline__ void chunk_sweep(
     const int32_t *__restrict__ seg_begin, const int32_t *__restrict__ segs,
@@ -2662,7 +2661,7 @@ static size_t sweep_smem(int w, int kind) {
     return w == 8 ? sweep_smem_bytes<8, kSweepWarps / 2>() : sweep_smem_bytes<4, kSweepWarps / 2>();
   return w == 8 ? sweep_smem_bytes<8, kSweepWarps>() : sweep_smem_bytes<4, kSweepWarps>();
 }
-// Cells of a warp's item in the deep sweeps.
+// Cells of a warp's item.
 static int32_t sweep_item_cells(int w) {
   return w == 8 ? SweepGeom<8>::kCells : SweepGeom<4>::kCells;
 }
@@ -2670,7 +2669,7 @@ static int32_t sweep_item_cells(int w) {
 struct ChunkSweep {
   int32_t *seg_begin = nullptr, *segs = nullptr;
   SweepNb *nbs = nullptr;
-  int32_t *seg_items = nullptr;  // warp items of the deep sweeps before each segment
+  int32_t *seg_items = nullptr;  // warp items before each segment
   PosCell *cells = nullptr;
   SweepRec *recs = nullptr;
   SweepRecF *recs_f = nullptr;  // mixed form
@@ -2737,7 +2736,7 @@ struct mfg_ctx {
   int32_t *bw_cells = nullptr, *bw_sptr = nullptr, *bw_nb = nullptr;
   SweepRec *bw_recs = nullptr;
   std::vector<int32_t> fw_lptr, bw_lptr;
-  // persistent sweeps: chunked level order, ready flags, error word
+  // persistent sweeps: chunked level order, increments, error word
   ChunkSweep fwc, bwc;
   int32_t nchunks = 0;
   bool chunk0_exported = false;
@@ -2745,7 +2744,7 @@ struct mfg_ctx {
   int *sweep_err = nullptr;
   int persist_grid = 0;
   int sweep_w = 0;               // records per position of the persistent sweeps (4 or 8)
-  int sweep_lanes = 0;           // lanes per cell of the persistent sweeps (= W)
+  int sweep_lanes = 0;           // mfg_set_sweep_lanes' value: W (a cell's lanes are W / 2)
   int persist_occ[2][2] = {{0, 0}, {0, 0}};  // resident blocks per SM [kind][W = 4, 8]
   int sweep_kind = MFG_SWEEP_DEEP;  // persistent sweep kernels in use (MFG_SWEEP_*)
   // launch knobs of the other kernels (mfg_autotune): resident blocks per SM
@@ -3180,7 +3179,6 @@ __global__ void k_dev_pack(int32_t C, int32_t W, int with_recs, const int32_t *_
     uint32_t e = (uint32_t)nb;
     int32_t slot = 0;
     if (cross) {
-      e |= kMark;
       atomicAdd(&stats[2], 1);
     } else if (nb < C && in_ring(posof[nb], segs[hscan[posof[nb]] + head[posof[nb]] - 1],
                                  seg_end, ring)) {
@@ -3922,7 +3920,6 @@ static int build_levels(mfg_ctx *ctx, const mfg_mesh *m, const std::vector<int32
                             in_ring(posof[nb], level_start[nb], seg_end, ctx->ring);
           if (nb < C && !ring) from_l2[fwd ? 0 : 1][nb] = 1;
           if (cross) {
-            e |= kMark;
             stat[2]++;
           } else if (ring) {
             e |= kInRing;
@@ -5375,8 +5372,9 @@ static int launch_bwd_persist(mfg_ctx *ctx, long long spin) {
 }
 
 // The sweeps' error word, on its way to pinned memory (fetch), then, once the
-// stream has been waited for, judged: on a timeout the flags are re-armed, so
-// that the context stays usable, and MFG_ERR_TIMEOUT is reported.
+// stream has been waited for, judged: on a timeout the forward increments are
+// armed again, so that the context stays usable, and MFG_ERR_TIMEOUT is
+// reported.
 static int fetch_sweep_error(mfg_ctx *ctx) {
   if (ctx->sweep_mode != 1) return MFG_OK;
   MFG_CUDA(cudaMemcpyAsync(ctx->h_pinned + 32, ctx->sweep_err, sizeof(int),
@@ -5466,7 +5464,7 @@ int mfg_forward_lusgs(mfg_ctx *ctx) {
 }
 
 // Failure-detection self-test: a forward sweep whose first chunk is never
-// run, so the cells that depend on it wait for flags nobody sets.  The
+// run, so the cells that depend on it wait for increments nobody writes.  The
 // bounded waits give up after spin_cycles; the call must return
 // MFG_ERR_TIMEOUT and leave the context usable.  State is not changed.
 int mfg_selftest_sweep_timeout(mfg_ctx *ctx, int64_t spin_cycles) {

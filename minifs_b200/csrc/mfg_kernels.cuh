@@ -169,16 +169,15 @@ __device__ __forceinline__ void store_q(double *__restrict__ q8, int64_t c, cons
   p[3] = make_double2(q[6], q[7]);
 }
 
-// Loads that must observe writes of earlier levels of the same sweep in a
-// persistent kernel: bypass the non-coherent path.
+// Loads that must observe writes of the sweep's earlier levels: bypass the
+// non-coherent path.
 __device__ __forceinline__ void load_dq_cg(const double *dq8, int64_t c, double *d) {
   const double2 *p = reinterpret_cast<const double2 *>(dq8 + c * Q_STRIDE);
   double2 a = __ldcg(p), b = __ldcg(p + 1), e = __ldcg(p + 2);
   d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y; d[4] = e.x;
 }
 
-// Plain (write-through) stores: readers in the same block see them after
-// __syncthreads, readers on other SMs through L2 after the release flag.
+// Plain (write-through) stores: later launches read them, through L2.
 __device__ __forceinline__ void store_dq(double *dq8, int64_t c, const double *d) {
   double2 *p = reinterpret_cast<double2 *>(dq8 + c * Q_STRIDE);
   p[0] = make_double2(d[0], d[1]);
@@ -652,11 +651,12 @@ __device__ __forceinline__ unsigned long long dbits(double x) {
 }
 
 // ---- readiness of LU-SGS increments -----------------------------------------
-// The forward and backward increments live in separate arrays whose interior
-// rows hold this signalling-NaN pattern until written.  IEEE arithmetic only
-// produces quiet NaNs, so a computed increment never equals it, and every
-// 8-byte word is written and read atomically: a reader may use a record as
-// soon as none of its five words is the sentinel, with no flag or fence.
+// The forward and backward increments live in separate arrays, in which the
+// rows that a sweep reads from L2 hold this signalling-NaN pattern until they
+// are written.  IEEE arithmetic only produces quiet NaNs, so a computed
+// increment never equals it, and every 8-byte word is written and read
+// atomically: a reader may use a record as soon as none of its five words is
+// the sentinel, with no flag or fence.
 constexpr unsigned long long kSentinelBits = 0x7FF40000DEADBEEFull;
 
 __device__ __forceinline__ bool is_sentinel(double x) {
@@ -684,8 +684,8 @@ __device__ __forceinline__ int ld_relaxed(const int *p) {
   return v;
 }
 
-// Cycles a lane may wait for one neighbour (~2 s at 1.9 GHz) before it gives
-// up, records the failure in *err and lets the sweep run to its end.
+// Cycles a lane may wait for one neighbour or level (~2 s at 1.9 GHz) before
+// it gives up and records the failure in *err, and the sweep ends.
 constexpr long long kSpinCycles = 4000000000LL;
 
 __device__ __forceinline__ void store_sentinel(double *dq8, int64_t c) {

@@ -166,7 +166,7 @@ class Solver:
         self._call("mfg_set_sweep_mode", int(mode))
 
     def set_sweep_lanes(self, lanes: int):
-        """Persistent sweeps: lanes per cell (the record slots per cell W)."""
+        """Takes the record slots per cell W only, and changes nothing."""
         self._call("mfg_set_sweep_lanes", int(lanes))
 
     def set_gather_lanes(self, lanes: int):
@@ -175,8 +175,9 @@ class Solver:
         self._call("mfg_set_gather_lanes", int(lanes))
 
     def autotune_sweeps(self, n_trial: int = 3) -> dict:
-        """Time both lane counts on this grid and keep the faster; the state
-        is left as it was.  Returns the choice and the ms per iteration."""
+        """Time fused iterations with the one value set_sweep_lanes takes; the
+        state is left as it was.  Returns it and the ms per iteration (-1 for
+        the value not taken); autotune times the launch parameters."""
         ms = np.zeros(2)
         self._call("mfg_autotune_sweeps", int(n_trial), int(self.iter_done), _lib.ptr(ms))
         info = self.info()
