@@ -293,8 +293,8 @@ int mfg_autotune(mfg_ctx *ctx, int32_t n_trial, int32_t iter_done, int32_t flags
  * usable (MFG_ERR_UNSUPPORTED when the grid has a single chunk). */
 int mfg_selftest_sweep_timeout(mfg_ctx *ctx, int64_t spin_cycles);
 /* Self-test of the division by a precomputed reciprocal, as the sweeps
- * divide by the diagonal and the gradient by a triangle's node count (no
- * counterpart in the reference): n pseudo-random dividend/divisor pairs
+ * divide by the diagonal and by a density and the gradient by a triangle's
+ * node count (no counterpart in the reference): n pseudo-random dividend/divisor pairs
  * (seeded, exponents across [-600, 600]; zero, subnormal and non-finite
  * dividends among them) divided both ways on the current device; *mismatches
  * receives the number of quotients whose bits differ from the division's,

@@ -1042,8 +1042,8 @@ k_sweep_bwd(int32_t l0, int32_t l1, const int32_t *__restrict__ cells,
 // memory for lane pairs of other warps, update by the producers; then whole
 // items per warp with the update in the sweep, a sentinel for every row, the
 // L2 increments polled before the level's wait and one level search per
-// level): 64^3 x 6 cells 511 / 565, 334 / 396, now 266 / 321; 128^3 3057 /
-// 3157 (blocks of two warps), -, 1577 / 2005; 16^3 117 / 132, 63 / 64, 52 /
+// level): 64^3 x 6 cells 511 / 565, 334 / 396, now 263 / 318; 128^3 3057 /
+// 3157 (blocks of two warps), -, 1568 / 1991; 16^3 117 / 132, 63 / 64, 51 /
 // 58.  Measured and not kept: thread-per-cell items (353 / 429), 14 or 16
 // warps of 128 registers (spills; 362 / 408), the item's rows by cp.async a
 // turn ahead (317 / 375: their shared-memory round trip loads the data pipe).
@@ -1230,14 +1230,12 @@ struct SweepIdx {
 };
 
 // What a lane keeps of one of its records: FP64, the neighbour-state half of
-// FluxLUSGS3D, the seed of its reciprocal, the normal out of the cell and the
-// weight; mixed, the neighbour's single-precision state, the normal and the
-// weight.
+// FluxLUSGS3D, the normal out of the cell and the weight; mixed, the
+// neighbour's single-precision state, the normal and the weight.
 template <bool MX>
 struct LaneRec {
   LusgsPre<double> a;
   double nx, ny, nz, w;
-  int seed;
 };
 template <>
 struct LaneRec<true> {
@@ -1256,7 +1254,7 @@ struct ChainP {
 __device__ __forceinline__ void lane_product(const LaneRec<false> &r, const double *DQ,
                                              const FluxP<double> &P, double *wf, int &bad) {
   double f[5];
-  flux_lusgs_fin_near(r.a, r.seed, DQ, r.nx, r.ny, r.nz, P, f, bad);
+  flux_lusgs_fin_near(r.a, DQ, r.nx, r.ny, r.nz, P, f, bad);
 #pragma unroll
   for (int k = 0; k < 5; k++) wf[k] = r.w * f[k];
 }
@@ -1473,11 +1471,9 @@ __device__ __forceinline__ void chunk_sweep(
           if (!has[u]) rec[u].nx = rec[u].ny = rec[u].nz = rec[u].w = 0.0f;
         } else {
           rec[u].a = flux_lusgs_pre(qn[u], rec[u].nx, rec[u].ny, rec[u].nz, FP);
-          rec[u].seed = rcp_seed(qn[u][0]);
           if (!has[u]) {
             rec[u] = LaneRec<MX>{};
             rec[u].a.Q0 = 1.0;
-            rec[u].seed = __double2hiint(1.0);
           }
         }
       };
@@ -2328,7 +2324,8 @@ __global__ void k_norm_seg_final(int32_t nparts, const double *__restrict__ part
 __global__ void k_counter_inc(int32_t *__restrict__ counter) { *counter += 1; }
 
 // Self-test of quot_near against the division, in the forms of the sweeps'
-// diagonal (a reciprocal that was divided for) and of a triangle's mean: n
+// diagonal (a reciprocal that was divided for), of a triangle's mean and of the
+// flux's density (rcp_rn_from, itself against 1 / b): n
 // dividend/divisor pairs from a splitmix64 stream, significands uniform,
 // exponents uniform in [-600, 600] (both sides of the window) and random
 // signs; every fourth divisor has an all-ones significand, three in 32
@@ -2369,15 +2366,24 @@ __global__ void k_selftest_division(int64_t n, uint64_t seed,
       const int e = (__double2hiint(v) >> 20) & 0x7FF;
       return e >= 1023 - 500 && e <= 1023 + 500;
     };
-    auto check = [&](double by, double y, int bad) {
-      const double q = quot_near(a, by, y, y, bad);
+    auto check = [&](double by, double near, double y, int bad) {
+      const double q = quot_near(a, by, near, y, bad);
       if ((bad >= 0) != ((a == 0.0 || inside(a)) && inside(by)))
         local++;
       else if (bad >= 0 && __double_as_longlong(q) != __double_as_longlong(a / by))
         local++;
     };
-    check(b, 1.0 / b, outside_exp(b, 523, 1523));
-    check(3.0, kRcp3, 0);
+    check(b, 1.0 / b, 1.0 / b, outside_exp(b, 523, 1523));
+    check(3.0, kRcp3, kRcp3, 0);
+    double near;
+    int bad_r = 0;
+    const double y = rcp_rn_from(b, rcp_approx(b), near, bad_r);
+    if ((bad_r >= 0) != (inside(b) && (i & 3) != 3))
+      local++;
+    else if (bad_r >= 0 && __double_as_longlong(y) != __double_as_longlong(1.0 / b))
+      local++;
+    else if (bad_r >= 0)
+      check(b, near, y, 0);
   }
   if (local) atomicAdd(bad, local);
 }
@@ -2417,7 +2423,7 @@ __global__ void k_selftest_functions(int mode, int32_t n, Params P, const double
     int bad = -1;
     if (mode == 3) {
       bad = 0;
-      flux_lusgs_fin_near(a, rcp_seed(q[0]), dq, c[10], c[11], c[12], fp, f, bad);
+      flux_lusgs_fin_near(a, dq, c[10], c[11], c[12], fp, f, bad);
     }
     if (bad < 0) flux_lusgs_fin(a, dq, c[10], c[11], c[12], fp, f);
     for (int k = 0; k < 5; k++) out[5 * (int64_t)i + k] = f[k];
@@ -2466,13 +2472,12 @@ __global__ void k_selftest_division_fast(int64_t n, uint64_t seed,
     int bady = 0;  // the gradient's form, by a volume
     const double q = quot_near(a, b, y, y, bady);
     if (bady < 0 || __double_as_longlong(q) != __double_as_longlong(a / b)) b1++;
-    // from the seed of a divisor within 1/16 of b
-    const double b0f = b * (1.0 + ((double)(int64_t)(ra >> 12) * 0x1p-52 - 0.5) * 0.115);
+    // the flux's form, by a density
     double near;
     int badn = 0, badq = 0, badz = 0;
-    const double yn = rcp_rn_near(b, __hiloint2double(rcp_seed(b0f), 0), near, badn);
+    const double yn = rcp_rn_from(b, rcp_approx(b), near, badn);
     if (badn < 0) {
-      if (fabs(b) > 0x1p-119 && fabs(b) < 0x1p119) b0++;  // inside the window
+      b0++;  // what rcp_rn_fast takes is inside the window
     } else {
       if (__double_as_longlong(yn) != __double_as_longlong(1.0 / b)) b0++;
       const double qn = quot_near(a, b, near, yn, badq);

@@ -43,28 +43,18 @@ __device__ __forceinline__ double quot_near(double a, double b, double near, dou
   return __hiloint2double((__double2hiint(q) & 0x7FFFFFFF) | sign, __double2loint(q));
 }
 
-// RN(1 / b) from an approximation y0 of it formed before b was known (the
-// sweeps': the reciprocal of the neighbour's density, b that density plus its
-// increment), for |e| < 1/16 with e = 1 - b y0.  The geometric series 1 / b =
-// y0 / (1 - e) = y0 (1 + e)(1 + e^2)(1 + e^4)(1 + O(e^8)) leaves 2^-32, a
-// Newton-Raphson step (`near`, within one ulp) and the final step of
-// rcp_rn_fast the rest: ten dependent operations instead of two conversions,
-// the hardware's approximation and six (61 against 138 cycles in one warp).
-// bad turns negative outside exponents of [-119, 119], for an all-ones
-// significand (as rcp_rn_fast's ok) and where e is larger.
-__device__ __forceinline__ double rcp_rn_near(double b, double y0, double &near, int &bad) {
-  const double e = __fma_rn(-b, y0, 1.0);
+// RN(1 / b) from an approximation y0 with e = 1 - b y0 of less than 2^-18: the
+// geometric series 1 / b = y0 / (1 - e) = y0 (1 + e + e^2 + O(e^3)) leaves
+// `near` within one ulp, and for such a reciprocal r = 1 - b near and RN(near +
+// near r) round correctly (Markstein, as above) except when the significand of
+// b is all ones.  bad turns negative for that significand and for an exponent
+// outside [-500, 500].
+__device__ __forceinline__ double rcp_rn_from(double b, double y0, double &near, int &bad) {
   const int ones = (__double2hiint(b) | 0xFFF00000) & __double2loint(b);
-  bad |= outside_exp(b, 1023 - 119, 1023 + 119) | (0x3FB00000 - 1 - hi_mag(e)) |
-         (ones == -1 ? -1 : 0);
-  const double e2 = __dmul_rn(e, e);
-  double y = __fma_rn(y0, e, y0);
-  const double e4 = __dmul_rn(e2, e2);
-  y = __fma_rn(y, e2, y);
-  y = __fma_rn(y, e4, y);
-  double r = __fma_rn(-b, y, 1.0);
-  near = __fma_rn(y, r, y);
-  r = __fma_rn(-b, near, 1.0);
+  bad |= outside_exp(b, 523, 1523) | (ones == -1 ? -1 : 0);
+  const double e = __fma_rn(-b, y0, 1.0);
+  near = __fma_rn(y0, __fma_rn(e, e, e), y0);
+  const double r = __fma_rn(-b, near, 1.0);
   return __fma_rn(near, r, near);
 }
 

@@ -47,16 +47,15 @@ static void quotient(double a, double b, double near, double y, int bad, bool b_
 }
 
 // a over b as the sweeps' diagonal, a triangle's mean, and the flux's density,
-// whose reciprocal starts from that of b (1 + off) in the high word
+// whose reciprocal starts from one that is off by the factor 1 + off
 static void check(double a, double b, double off) {
   quotient(a, b, 1.0 / b, 1.0 / b, mfg::outside_exp(b, 523, 1523), within(b, 500));
   quotient(a, 3.0, 1.0 / 3.0, 1.0 / 3.0, 0, true);
-  const double seed = number(bits((double)(float)(1.0 / (b * (1.0 + off)))) >> 32 << 32);
   double near = 0.0;
   int bad = 0;
-  const double y = mfg::rcp_rn_near(b, seed, near, bad);
+  const double y = mfg::rcp_rn_from(b, 1.0 / b * (1.0 + off), near, bad);
   const bool ones = (bits(b) & 0xFFFFFFFFFFFFFull) == 0xFFFFFFFFFFFFFull;
-  if ((bad >= 0) != (within(b, 119) && !ones)) wrong_side++;
+  if ((bad >= 0) != (within(b, 500) && !ones)) wrong_side++;
   if (bad < 0) return;
   if (bits(y) != bits(1.0 / b)) wrong_r++;
   quotient(a, b, near, y, 0, true);
@@ -83,7 +82,8 @@ int main(int argc, char **argv) {
         for (uint64_t mb : mant)
           for (int s = 0; s < 4; s++)
             check(number((uint64_t)(s & 1) << 63 | (uint64_t)ea << 52 | ma),
-                  number((uint64_t)(s >> 1) << 63 | (uint64_t)eb << 52 | mb), 0.0);
+                  number((uint64_t)(s >> 1) << 63 | (uint64_t)eb << 52 | mb),
+                  s & 1 ? 0x1.fp-19 : -0x1.fp-19);
   for (long long i = 0; i < n; i++) {
     const uint64_t r = splitmix64(&x), e = splitmix64(&x), t = splitmix64(&x), o = splitmix64(&x);
     const uint64_t ea = 1023 - 600 + e % 1201;
@@ -91,7 +91,7 @@ int main(int argc, char **argv) {
     uint64_t mb = t & 0xFFFFFFFFFFFFFull;
     if ((i & 6) == 6) mb = 0xFFFFFFFFFFFFFull - (i >> 3 & 1);
     check(number((r >> 63) << 63 | ea << 52 | (r & 0xFFFFFFFFFFFFFull)),
-          number((t >> 63) << 63 | eb << 52 | mb), ((double)(o >> 11) * 0x1p-53 - 0.5) * 0.115);
+          number((t >> 63) << 63 | eb << 52 | mb), ((double)(o >> 11) * 0x1p-53 - 0.5) * 0x1.fcp-18);
   }
   printf("%lld %lld %lld\n", wrong_q, wrong_r, wrong_side);
   return 0;
